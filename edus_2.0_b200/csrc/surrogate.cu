@@ -248,6 +248,666 @@ __global__ void adam_kernel(float* __restrict__ w, __nv_bfloat16* __restrict__ w
     }
 }
 
+// ---------------------------------------------------------------------------
+// Networks of hidden width 128 (what the surrogate uses): the whole forward
+// and backward chain of 128 batch rows in one CTA, the weight gradients in one
+// grouped split-K launch, reduction and Adam in a third.
+//
+// Layer by layer through global memory this step was bound by its launches and
+// by serial work, not by arithmetic: the weight gradients contract over the
+// batch, so each was one CTA walking 4096 rows (0.88 ms a layer), and the
+// column sums were one thread a column (0.23 ms); 4096 x 259 -> 254 took
+// 4.05 ms a training step.  Here activations never leave the SM between
+// layers (shared memory as BF16 operands, tensor memory as FP32
+// pre-activations), and each layer's gradient is spread over the SMs by tiles and
+// column groups.
+//
+// Operand blocks.  Activations, gradients and weights are 128 x 128 BF16 blocks
+// (32 KB) of 8 x 8 core matrices (128 B).  Gradients and weights: element (r, c)
+// at (r >> 3) * 1024 + (c >> 3) * 64 + (r & 7) * 8 + (c & 7).  Read with c along K
+// this is the K-major operand layout (core matrices 128 B apart along K, 2048 B
+// along the rows); read with r along K it is the MN-major layout of the
+// transposed matrix.  Activations: four column groups of 32, each laid out that
+// way (512 B between row groups), so that a group is contiguous.  One copy of
+// each block therefore serves both products it enters: an activation block (r =
+// batch row, c = feature) is the row operand of the forward product and, by
+// column groups, the column operand of the weight gradient; a weight block (r =
+// output, c = input) is used as it is forward and transposed backward.  Blocks
+// move between global and shared memory by bulk copies.
+constexpr int kBlk = 128 * 128;            // elements of a block
+constexpr unsigned kBlkBytes = kBlk * 2u;  // 32 KB
+constexpr int kGrp = 128 * 32;             // elements of an activation block's column group
+constexpr int kRing = 3;                   // weight blocks in flight
+constexpr int kActs = 3;                   // activation blocks in shared memory
+constexpr size_t kRowsSmem = (size_t)(kRing + kActs) * kBlkBytes + 1024;
+constexpr int kDwStages = 5;
+constexpr unsigned kDwStage = kBlkBytes + kGrp * 2u;  // a dz block and an activation column group
+constexpr size_t kDwSmem = (size_t)kDwStages * kDwStage + 1024;
+constexpr unsigned kBiasStage = 128 * 32 * 4;  // 128 rows x 32 outputs of dz in FP32
+constexpr int kMlpPolls = 1 << 22;
+
+__device__ __forceinline__ int blk_off(int r, int c) { return (r >> 3) * 1024 + (c >> 3) * 64 + (r & 7) * 8 + (c & 7); }
+__device__ __forceinline__ int act_off(int r, int c) {
+    return (c >> 5) * kGrp + (r >> 3) * 256 + ((c >> 3) & 3) * 64 + (r & 7) * 8 + (c & 7);
+}
+
+// operand descriptor: `kcore` bytes between core matrices along K, `mncore` along the rows
+__device__ __forceinline__ unsigned long long op_desc(const void* p, unsigned kcore, unsigned mncore) {
+    return (unsigned long long)((smem_addr(p) >> 4) & 0x3FFFu) | ((unsigned long long)(kcore >> 4) << 16) |
+           ((unsigned long long)(mncore >> 4) << 32) | (1ull << 46);
+}
+__device__ __forceinline__ void mma_k16(unsigned tmem, unsigned long long da, unsigned long long db, unsigned idesc, bool accumulate) {
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
+        "l"(da), "l"(db), "r"(idesc), "r"(accumulate ? 1u : 0u)
+        : "memory");
+}
+constexpr unsigned kTransA = 1u << 15, kTransB = 1u << 16;
+
+// acc[128][128] (+)= A W^T or A W over a block's K of 128 (8 MMAs of K = 16), by
+// one thread.  A: an activation block (ACT) or a gradient block, K along its
+// columns; W: a weight block, K along its columns (forward) or rows (backward).
+template <bool ACT, bool FORWARD>
+__device__ __forceinline__ void rows_mma(const __nv_bfloat16* A, const __nv_bfloat16* W, unsigned tmem, bool accumulate) {
+#pragma unroll
+    for (int st = 0; st < 8; ++st) {
+        const unsigned long long da = ACT ? op_desc(A + (st >> 1) * kGrp + (st & 1) * 128, 128, 512)
+                                          : op_desc(A + st * 128, 128, 2048);
+        const unsigned long long db = FORWARD ? op_desc(W + st * 128, 128, 2048) : op_desc(W + st * 2048, 2048, 128);
+        mma_k16(tmem, da, db, kUmmaIdesc | (FORWARD ? 0u : kTransB), accumulate || st > 0);
+    }
+}
+// acc[out 128][in 32] (+)= dz^T act over 128 batch rows: both operands MN-major
+__device__ __forceinline__ void dw_mma(const __nv_bfloat16* dz, const __nv_bfloat16* act, unsigned tmem, bool accumulate) {
+    constexpr unsigned idesc =
+        (1u << 4) | (1u << 7) | (1u << 10) | kTransA | kTransB | ((32u >> 3) << 17) | ((unsigned)(UM >> 4) << 24);
+#pragma unroll
+    for (int st = 0; st < 8; ++st)
+        mma_k16(tmem, op_desc(dz + st * 2048, 2048, 128), op_desc(act + st * 512, 512, 128), idesc,
+                accumulate || st > 0);
+}
+__device__ __forceinline__ void mma_commit(unsigned long long* bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(smem_addr(bar))
+                 : "memory");
+}
+__device__ __forceinline__ void bar_init1(unsigned long long* bar) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_addr(bar)) : "memory");
+}
+// block global -> shared, completion on bar (which takes one arrival per copy)
+__device__ __forceinline__ void blk_load(void* dst, const void* src, unsigned long long* bar, unsigned bytes = kBlkBytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_addr(bar)), "r"(bytes)
+                 : "memory");
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
+                     smem_addr(dst)),
+                 "l"(reinterpret_cast<unsigned long long>(src)), "r"(bytes), "r"(smem_addr(bar))
+                 : "memory");
+}
+// 32 KB block shared -> global, one bulk group of the issuing thread
+__device__ __forceinline__ void blk_store(void* dst, const void* src) {
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n" ::"l"(
+                     reinterpret_cast<unsigned long long>(dst)),
+                 "r"(smem_addr(src)), "r"(kBlkBytes)
+                 : "memory");
+    asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
+}
+__device__ __forceinline__ void tmem_ld16(float* v, unsigned addr) {
+    unsigned u[16];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, "
+        "[%16];\n"
+        : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7]), "=r"(u[8]),
+          "=r"(u[9]), "=r"(u[10]), "=r"(u[11]), "=r"(u[12]), "=r"(u[13]), "=r"(u[14]), "=r"(u[15])
+        : "r"(addr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(u[i]);
+}
+// 16 consecutive columns of row r of an activation (ACT) or gradient block, rounded to BF16
+template <bool ACT>
+__device__ __forceinline__ void blk_put16(__nv_bfloat16* blk, int r, int c, const float* v) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        __nv_bfloat162 p[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) p[i] = __floats2bfloat162_rn(v[8 * h + 2 * i], v[8 * h + 2 * i + 1]);
+        *reinterpret_cast<uint4*>(blk + (ACT ? act_off(r, c + 8 * h) : blk_off(r, c + 8 * h))) = *reinterpret_cast<uint4*>(p);
+    }
+}
+// v[i] of lane j <-> v[j] of lane i over the warp
+__device__ __forceinline__ void warp_transpose32(float* v, int lane) {
+#pragma unroll
+    for (int s = 16; s >= 1; s >>= 1) {
+        const bool up = lane & s;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+            if (i & s) continue;
+            const float got = __shfl_xor_sync(0xffffffffu, up ? v[i] : v[i + s], s);
+            if (up) v[i] = got;
+            else v[i + s] = got;
+        }
+    }
+}
+
+struct MlpRowsArgs {
+    int B, n_in, n_out, KT, NT;
+    const float* x;            // [B][n_in]
+    const float* t;            // [B][n_out] (TRAIN)
+    float* y;                  // [B][n_out] (forward only)
+    const __nv_bfloat16* wp;   // weight blocks: layer 0 by input block, layers 1, 2, output layer by output block
+    const float* bias[4];
+    __nv_bfloat16* act;        // [row block][KT + 3]: x blocks, a1, a2, a3 (TRAIN)
+    __nv_bfloat16* dz;         // [row block][3 + NT]: dz of layers 0, 1, 2 and of the output blocks (TRAIN)
+    float* dzf;                // [row block][3 + NT][4 column groups][128][32]: dz in FP32 (TRAIN)
+    float* lossp;              // [row block] (TRAIN)
+    float scale;               // 1 / (B n_out)
+    int* status;
+};
+
+// 128 batch rows through the network and, with TRAIN, back.  16 warps; warp w
+// reads tensor-memory lanes 32 (w & 3) .. + 31 (its rows) and the 32 columns from
+// 32 (w >> 2).  Tensor-memory columns: the pre-activations of the three hidden
+// layers at 0, 128, 256, the output block at 384; backward, the gradient of a
+// layer's activations takes the columns of the layer above it.  Every wait is
+// bounded; one that runs out sets *status and ends the CTA.
+template <bool TRAIN>
+__global__ void __launch_bounds__(512, 1) mlp_rows_kernel(MlpRowsArgs a) {
+    extern __shared__ unsigned char mraw[];
+    __shared__ __align__(8) unsigned long long full[kRing], mma_bar, rel_bar;
+    __shared__ unsigned tmem_slot;
+    __shared__ int failed;
+    __shared__ float red[16];
+    __nv_bfloat16* act = (__nv_bfloat16*)(((unsigned long long)mraw + 1023) & ~1023ull);
+    __nv_bfloat16* ring = act + kActs * kBlk;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int row = (warp & 3) * 32 + lane, col0 = (warp >> 2) * 32;
+    const int grow = blockIdx.x * 128 + row;
+    const bool live = grow < a.B;
+    const int KT = a.KT, NT = a.NT;
+    const int nqf = KT + 2 + NT, nq = TRAIN ? nqf + NT + 2 : nqf;
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_addr(&tmem_slot)),
+                     "r"(512)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+    }
+    // weight block of product q (forward layers, then backward from the output)
+    auto wblock = [&](int q) {
+        if (q < nqf) return q;
+        const int p = q - nqf;
+        return p < NT ? KT + 2 + p : (p == NT ? KT + 1 : KT);
+    };
+    int issued = 0;  // thread 0: weight blocks requested
+    auto prefetch = [&](int q) {
+        if (q < nq) {
+            blk_load(ring + (q % kRing) * kBlk, a.wp + (size_t)wblock(q) * kBlk, &full[q % kRing]);
+            issued = q + 1;
+        }
+    };
+    if (tid == 0) {
+        failed = 0;
+        for (int i = 0; i < kRing; ++i) bar_init1(&full[i]);
+        bar_init1(&mma_bar);
+        bar_init1(&rel_bar);
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+        for (int q = 0; q < kRing; ++q) prefetch(q);
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    const unsigned tmem = tmem_slot;
+    const unsigned lanes = tmem + ((unsigned)((warp & 3) * 32) << 16);
+
+    // product q: A block (written by this CTA) times the weight block; the
+    // A block also goes to `keep` in global memory for the weight gradients
+    auto product = [&](int q, const __nv_bfloat16* A, bool forward, unsigned col, bool accumulate, __nv_bfloat16* keep) {
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+        // stores older than the last one have left their buffers
+        if (TRAIN && tid == 0) asm volatile("cp.async.bulk.wait_group.read 1;\n" ::: "memory");
+        __syncthreads();
+        if (tid == 0) {
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+            if (!mbar_wait_parity(&full[q % kRing], (unsigned)((q / kRing) & 1), kMlpPolls)) failed = 1;
+            const __nv_bfloat16* W = ring + (q % kRing) * kBlk;
+            if (forward) rows_mma<true, true>(A, W, tmem + col, accumulate);
+            else rows_mma<false, false>(A, W, tmem + col, accumulate);
+            mma_commit(&mma_bar);
+            if (TRAIN && keep) blk_store(keep, A);
+        }
+    };
+    // product q is done (all threads agree); its weight block's slot is refilled
+    auto finished = [&](int q) {
+        const bool ok = mbar_wait_parity(&mma_bar, (unsigned)(q & 1), kMlpPolls);
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        if (__syncthreads_or(!ok || failed)) return false;
+        if (tid == 0) prefetch(q + kRing);
+        return true;
+    };
+    __nv_bfloat16* keep_act = TRAIN ? a.act + (size_t)blockIdx.x * (KT + 3) * kBlk : nullptr;
+    __nv_bfloat16* keep_dz = TRAIN ? a.dz + (size_t)blockIdx.x * (3 + NT) * kBlk : nullptr;
+    bool ok = true;
+    int nblk = 0;  // activation blocks written so far: block i sits in buffer i % kActs
+    auto buffer = [&](int i) { return act + (i % kActs) * kBlk; };
+
+    // 128 rows x 128 input features, FP32 to BF16 (a warp's 32 loads a lane are
+    // in flight together); rows and features past the ends are zero
+    auto load_x = [&](int kt, __nv_bfloat16* dst) {
+        const int r0 = warp * 8;
+        float v[8][4];
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            const long long gr = (long long)blockIdx.x * 128 + r0 + r;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int c = kt * 128 + lane + 32 * j;
+                v[r][j] = (gr < a.B && c < a.n_in) ? __ldg(a.x + gr * a.n_in + c) : 0.f;
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < 8; ++r)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) dst[act_off(r0 + r, lane + 32 * j)] = __float2bfloat16(v[r][j]);
+    };
+    // the warp's 32 x 32 of dz in FP32, for the bias gradients (v is spent)
+    auto put_dzf = [&](float* v, int slot) {
+        warp_transpose32(v, lane);
+        float* d = a.dzf + ((((size_t)blockIdx.x * (3 + NT) + slot) * 4 + (warp >> 2)) * 128 + (warp & 3) * 32) * 32 + lane;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) d[i * 32] = v[i];
+    };
+
+    int q = 0;
+    load_x(0, buffer(nblk));
+    for (int kt = 0; ok && kt < KT; ++kt, ++q) {
+        product(q, buffer(nblk), true, 0, kt > 0, TRAIN ? keep_act + (size_t)kt * kBlk : nullptr);
+        ++nblk;
+        if (kt + 1 < KT) load_x(kt + 1, buffer(nblk));
+        ok = finished(q);
+    }
+    for (int l = 0; ok && l < 3; ++l) {
+        __nv_bfloat16* dst = buffer(nblk++);
+#pragma unroll 1
+        for (int c0 = col0; c0 < col0 + 32; c0 += 16) {
+            float v[16];
+            tmem_ld16(v, lanes + l * 128 + c0);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] = gelu(v[i] + __ldg(&a.bias[l][c0 + i]));
+            blk_put16<true>(dst, row, c0, v);
+        }
+        if (l < 2) {
+            product(q, dst, true, (l + 1) * 128, false, TRAIN ? keep_act + (size_t)(KT + l) * kBlk : nullptr);
+            ok = finished(q++);
+        }
+    }
+    const __nv_bfloat16* a3 = buffer(nblk - 1);
+    const int b3 = nblk - 1;
+    float loss = 0.f;
+    for (int nt = 0; ok && nt < NT; ++nt) {
+        // the warp's 32 x 32 targets, row by row (coalesced), before the product's wait
+        const int col = nt * 128 + col0;
+        const long long wrow = (long long)blockIdx.x * 128 + (warp & 3) * 32;
+        float tv[32];
+        if (TRAIN) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+                tv[i] = (wrow + i < a.B && col + lane < a.n_out) ? __ldg(a.t + (wrow + i) * a.n_out + col + lane) : 0.f;
+        }
+        product(q, a3, true, 384, false, (TRAIN && nt == 0) ? keep_act + (size_t)(KT + 2) * kBlk : nullptr);
+        ok = finished(q++);
+        if (!ok) break;
+        // output blocks take turns in the two buffers that a3 leaves; an earlier
+        // block's store has left its buffer (product() waited for it)
+        __nv_bfloat16* dst = buffer(b3 + 1 + (nt & 1));
+        float v[32];
+        tmem_ld16(v, lanes + 384 + col0);
+        tmem_ld16(v + 16, lanes + 384 + col0 + 16);
+        if (TRAIN) {
+            warp_transpose32(tv, lane);
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+                const bool on = live && col + i < a.n_out;
+                const float d = on ? v[i] + __ldg(&a.bias[3][col + i]) - tv[i] : 0.f;
+                loss += d * d;
+                v[i] = 2.f * d * a.scale;
+            }
+            blk_put16<false>(dst, row, col0, v);
+            blk_put16<false>(dst, row, col0 + 16, v + 16);
+            put_dzf(v, 3 + nt);
+        } else {
+            warp_transpose32(v, lane);
+            const float bias = col + lane < a.n_out ? __ldg(&a.bias[3][col + lane]) : 0.f;
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+                if (wrow + i < a.B && col + lane < a.n_out) a.y[(wrow + i) * a.n_out + col + lane] = v[i] + bias;
+        }
+        if (TRAIN) {
+            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+            __syncthreads();
+            if (tid == 0) {
+                blk_store(keep_dz + (size_t)(3 + nt) * kBlk, dst);
+                // the other buffer is free before the next block is written there
+                asm volatile("cp.async.bulk.wait_group.read 1;\n" ::: "memory");
+            }
+        }
+    }
+    if (TRAIN) {
+        __syncthreads();
+        if (ok) {
+            // loss of these rows
+#pragma unroll
+            for (int s = 16; s > 0; s >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, s);
+            if (lane == 0) red[warp] = loss;
+            __syncthreads();
+            if (tid == 0) {
+                float s = 0.f;
+                for (int i = 0; i < 16; ++i) s += red[i];
+                a.lossp[blockIdx.x] = s * a.scale;
+            }
+        }
+        // gradient of a3: sum over the output blocks of dz_out W^T (columns 384; more
+        // than two blocks are read back from global memory)
+        int nrel = 0;
+        for (int nt = 0; ok && nt < NT; ++nt) {
+            const __nv_bfloat16* A = buffer(b3 + 1 + (nt & 1));
+            if (NT > 2) {
+                if (tid == 0) {
+                    asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory");  // the blocks are written
+                    blk_load(act + (size_t)((b3 + 1 + (nt & 1)) % kActs) * kBlk, keep_dz + (size_t)(3 + nt) * kBlk, &rel_bar);
+                }
+                const bool got = mbar_wait_parity(&rel_bar, (unsigned)(nrel & 1), kMlpPolls);
+                ++nrel;
+                if (__syncthreads_or(!got)) {
+                    ok = false;
+                    break;
+                }
+            }
+            product(q, A, false, 384, nt > 0, nullptr);
+            ok = finished(q++);
+        }
+        nblk = b3 + 3;  // the next buffer is a3's, whose products and store are done
+        for (int l = 2; ok && l >= 0; --l) {
+            // dz_l = da * GELU'(z_l): da in columns (l + 1) * 128, z_l in l * 128
+            if (tid == 0) asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");
+            __syncthreads();
+            __nv_bfloat16* dst = buffer(nblk++);
+            float v[32];
+#pragma unroll
+            for (int c0 = 0; c0 < 32; c0 += 16) {
+                float z[16];
+                tmem_ld16(v + c0, lanes + (l + 1) * 128 + col0 + c0);
+                tmem_ld16(z, lanes + l * 128 + col0 + c0);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) v[c0 + i] *= gelu_grad(z[i] + __ldg(&a.bias[l][col0 + c0 + i]));
+                blk_put16<false>(dst, row, col0 + c0, v + c0);
+            }
+            put_dzf(v, l);
+            if (l > 0) {
+                product(q, dst, false, l * 128, false, keep_dz + (size_t)l * kBlk);
+                ok = finished(q++);
+            } else {
+                asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+                __syncthreads();
+                if (tid == 0) blk_store(keep_dz, dst);
+            }
+        }
+    }
+    if (tid == 0) {
+        if (!ok) {
+            atomicOr(a.status, 1);
+            // weight blocks still in flight land before the CTA ends
+            for (int i = issued - 1; i >= 0 && i >= issued - kRing; --i)
+                mbar_wait_parity(&full[i % kRing], (unsigned)((i / kRing) & 1), kMlpPolls);
+        }
+        asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(512) : "memory");
+}
+
+// Weight gradients: CTA (tile, group) contracts over the whole batch in row
+// order, grad[tile][c][r] = sum over rows of act(row, c) dz(row, r), for 32 of
+// the tile's 128 inputs c (r = output, c = input of one layer's 128 x 128 tile).
+// The batch is not split: the sums are those of one accumulator that walks the
+// rows, at 40 KB a row block, which five stages of copies keep flowing.
+//
+// blockIdx.x past the tiles: the bias gradients of 32 outputs (slot of dz, column
+// group blockIdx.y), one lane an output, summed in row order; 16 KB a row block.
+__global__ void __launch_bounds__(128, 1) mlp_dw_kernel(const __nv_bfloat16* __restrict__ act,
+                                                        const __nv_bfloat16* __restrict__ dz,
+                                                        const float* __restrict__ dzf, int KT, int NT, int nrb, int B,
+                                                        float* __restrict__ grad, float* __restrict__ bgrad,
+                                                        int* __restrict__ status) {
+    extern __shared__ unsigned char mraw[];
+    __shared__ __align__(8) unsigned long long full[kDwStages], read[kDwStages], done;
+    __shared__ unsigned tmem_slot;
+    unsigned char* buf = (unsigned char*)(((unsigned long long)mraw + 1023) & ~1023ull);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tile = blockIdx.x, grp = blockIdx.y;
+    if (tile >= KT + 2 + NT) {
+        if (warp) return;
+        const int slot = tile - (KT + 2 + NT);
+        if (lane == 0) {
+            for (int i = 0; i < kDwStages; ++i) bar_init1(&full[i]);
+            asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+        }
+        __syncwarp();
+        auto load = [&](int i) {
+            blk_load(buf + (size_t)(i % kDwStages) * kBiasStage,
+                     dzf + (((size_t)i * (3 + NT) + slot) * 4 + grp) * (128 * 32), &full[i % kDwStages], kBiasStage);
+        };
+        int loaded = 0;
+        if (lane == 0)
+            for (; loaded < nrb && loaded < kDwStages; ++loaded) load(loaded);
+        float sum = 0.f;
+        bool ok = true;
+        int i = 0;
+        for (; ok && i < nrb; ++i) {
+            ok = __all_sync(0xffffffffu, mbar_wait_parity(&full[i % kDwStages], (unsigned)((i / kDwStages) & 1), kMlpPolls));
+            if (!ok) break;
+            const float* d = (const float*)(buf + (size_t)(i % kDwStages) * kBiasStage) + lane;
+            const int rows = min(128, B - i * 128);
+            int r = 0;
+            for (; r + 16 <= rows; r += 16) {
+                float x[16];
+#pragma unroll
+                for (int j = 0; j < 16; ++j) x[j] = d[(r + j) * 32];
+#pragma unroll
+                for (int j = 0; j < 16; ++j) sum += x[j];
+            }
+            for (; r < rows; ++r) sum += d[r * 32];
+            __syncwarp();
+            if (lane == 0 && loaded < nrb) load(loaded++);
+        }
+        if (ok) bgrad[slot * 128 + grp * 32 + lane] = sum;
+        else if (lane == 0) {
+            atomicOr(status, 1);
+            for (int j = i; j < loaded; ++j)
+                mbar_wait_parity(&full[j % kDwStages], (unsigned)((j / kDwStages) & 1), kMlpPolls);
+        }
+        return;
+    }
+    const int ablk = tile < KT + 2 ? tile : KT + 2;
+    const int zblk = tile < KT ? 0 : (tile < KT + 2 ? tile - KT + 1 : 3 + tile - KT - 2);
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_addr(&tmem_slot)),
+                     "r"(32)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+    }
+    if (tid == 0) {
+        for (int i = 0; i < kDwStages; ++i) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 2;\n" ::"r"(smem_addr(&full[i])) : "memory");
+            bar_init1(&read[i]);
+        }
+        bar_init1(&done);
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    const unsigned tmem = tmem_slot;
+    bool ok = true;
+    if (tid == 0) {
+        auto load = [&](int i) {
+            unsigned char* d = buf + (size_t)(i % kDwStages) * kDwStage;
+            blk_load(d, dz + ((size_t)i * (3 + NT) + zblk) * kBlk, &full[i % kDwStages]);
+            blk_load(d + kBlkBytes, act + ((size_t)i * (KT + 3) + ablk) * kBlk + grp * kGrp, &full[i % kDwStages],
+                     kGrp * 2u);
+        };
+        int loaded = 0, used = 0;
+        for (; loaded < nrb && loaded < kDwStages; ++loaded) load(loaded);
+        for (; ok && used < nrb; ++used) {
+            const int i = used;
+            ok = mbar_wait_parity(&full[i % kDwStages], (unsigned)((i / kDwStages) & 1), kMlpPolls);
+            if (!ok) break;
+            const __nv_bfloat16* d = (const __nv_bfloat16*)(buf + (size_t)(i % kDwStages) * kDwStage);
+            dw_mma(d, d + kBlk, tmem, i > 0);
+            mma_commit(&read[i % kDwStages]);
+            // the stage that the previous row block has left takes a new one
+            if (i >= 1 && loaded < nrb) {
+                ok = mbar_wait_parity(&read[(i - 1) % kDwStages], (unsigned)(((i - 1) / kDwStages) & 1), kMlpPolls);
+                if (ok) load(loaded++);
+            }
+        }
+        if (!ok) {
+            atomicOr(status, 1);
+            for (int j = used; j < loaded; ++j)  // no copy may land after the CTA ends
+                mbar_wait_parity(&full[j % kDwStages], (unsigned)((j / kDwStages) & 1), kMlpPolls);
+        }
+        mma_commit(&done);
+    }
+    ok = mbar_wait_parity(&done, 0, kMlpPolls) && ok;
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    if (!__syncthreads_or(!ok)) {
+        // lane = output, tensor-memory column = input: each column is a coalesced row of the tile
+        float* dst = grad + (size_t)tile * kBlk + (size_t)grp * 32 * 128 + warp * 32 + lane;
+#pragma unroll 1
+        for (int c0 = 0; c0 < 32; c0 += 16) {
+            float v[16];
+            tmem_ld16(v, tmem + ((unsigned)(warp * 32) << 16) + c0);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) dst[(c0 + i) * 128] = v[i];
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(32) : "memory");
+}
+
+// Where parameter i lives: layer, weight (input k, output n) or bias (k = -1).
+struct MlpShape {
+    int n_in, n_out, KT, NT;
+    long long woff[4], boff[4];
+    long long nparams;
+};
+__device__ __forceinline__ void mlp_locate(const MlpShape& s, long long i, int& l, int& k, int& n) {
+    l = i < s.woff[1] ? 0 : (i < s.woff[2] ? 1 : (i < s.woff[3] ? 2 : 3));
+    const long long wo = l == 0 ? s.woff[0] : (l == 1 ? s.woff[1] : (l == 2 ? s.woff[2] : s.woff[3]));
+    const long long bo = l == 0 ? s.boff[0] : (l == 1 ? s.boff[1] : (l == 2 ? s.boff[2] : s.boff[3]));
+    const int out = l < 3 ? 128 : s.n_out;
+    if (i >= bo) {
+        k = -1;
+        n = (int)(i - bo);
+    } else {
+        const int e = (int)(i - wo);
+        k = e / out;
+        n = e - k * out;
+    }
+}
+// block index of weight (l, k, n) and its row (output) and column (input) there
+__device__ __forceinline__ int mlp_block(const MlpShape& s, int l, int k, int n, int& r, int& c) {
+    r = n & 127;
+    c = k & 127;
+    return l == 0 ? (k >> 7) : (l < 3 ? s.KT + l - 1 : s.KT + 2 + (n >> 7));
+}
+
+// BF16 weight blocks from the FP32 parameters (padding stays zero from the allocation)
+__global__ void mlp_pack_kernel(MlpShape s, const float* __restrict__ w, __nv_bfloat16* __restrict__ wp) {
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < s.nparams; i += (long long)gridDim.x * blockDim.x) {
+        int l, k, n, r, c;
+        mlp_locate(s, i, l, k, n);
+        if (k < 0) continue;
+        const int b = mlp_block(s, l, k, n, r, c);
+        wp[(size_t)b * kBlk + blk_off(r, c)] = __float2bfloat16(w[i]);
+    }
+}
+
+// The gradients in parameter order and, with lr > 0, the Adam update of the
+// master weights and their BF16 blocks.  Blocks 0 .. 8 tiles - 1: a thread takes
+// eight inputs of one output of a weight tile, so its BF16 weights are one 16-byte
+// row of a core matrix and neighbouring threads read neighbouring outputs (one
+// parameter a thread, with 2-byte stores into the blocks, took 18 us for 99 k
+// parameters; this way 12).  The next blocks: a thread per bias; the last sums the loss.
+struct AdamArgs {
+    float lr, b1, b2, eps, c1, c2;
+};
+__device__ __forceinline__ float adam_step(const AdamArgs& ad, float g, float* w, float* m, float* v) {
+    const float mi = ad.b1 * *m + (1.f - ad.b1) * g;
+    const float vi = ad.b2 * *v + (1.f - ad.b2) * g * g;
+    *m = mi;
+    *v = vi;
+    const float wi = *w - ad.lr * (mi / ad.c1) / (sqrtf(vi / ad.c2) + ad.eps);
+    *w = wi;
+    return wi;
+}
+__global__ void __launch_bounds__(256) mlp_update_kernel(MlpShape s, const float* __restrict__ dw,
+                                                         const float* __restrict__ bgrad,
+                                                         const float* __restrict__ lossp, int nrb,
+                                                         float* __restrict__ grads, float* __restrict__ w,
+                                                         __nv_bfloat16* __restrict__ wp, float* __restrict__ m,
+                                                         float* __restrict__ v, float* __restrict__ loss, AdamArgs ad) {
+    const int tiles = s.KT + 2 + s.NT;
+    if ((int)blockIdx.x < 8 * tiles) {
+        const int tile = blockIdx.x >> 3;
+        const int r = threadIdx.x & 127, c0 = ((blockIdx.x & 7) * 2 + (threadIdx.x >> 7)) * 8;
+        const int l = tile < s.KT ? 0 : (tile < s.KT + 2 ? tile - s.KT + 1 : 3);
+        const int k0 = (l == 0 ? tile * 128 : 0) + c0, n = (l == 3 ? (tile - s.KT - 2) * 128 : 0) + r;
+        const int in = l == 0 ? s.n_in : 128, out = l == 3 ? s.n_out : 128;
+        if (n >= out) return;
+        const long long wo = l == 0 ? s.woff[0] : (l == 1 ? s.woff[1] : (l == 2 ? s.woff[2] : s.woff[3]));
+        float g[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) g[j] = dw[(size_t)tile * kBlk + (c0 + j) * 128 + r];
+        float wi[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            wi[j] = 0.f;
+            if (k0 + j < in) {
+                const long long i = wo + (long long)(k0 + j) * out + n;
+                grads[i] = g[j];
+                if (ad.lr > 0.f) wi[j] = adam_step(ad, g[j], w + i, m + i, v + i);
+            }
+        }
+        if (ad.lr > 0.f) {
+            __nv_bfloat162 p[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) p[j] = __floats2bfloat162_rn(wi[2 * j], wi[2 * j + 1]);
+            *reinterpret_cast<uint4*>(wp + (size_t)tile * kBlk + blk_off(r, c0)) = *reinterpret_cast<uint4*>(p);
+        }
+        return;
+    }
+    if (blockIdx.x == gridDim.x - 1) {
+        if (threadIdx.x >= 32) return;
+        float t = 0.f;
+        for (int i = threadIdx.x; i < nrb; i += 32) t += lossp[i];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (threadIdx.x == 0) *loss = t;
+        return;
+    }
+    const int q = ((int)blockIdx.x - 8 * tiles) * 256 + threadIdx.x;
+    if (q >= 384 + s.n_out) return;
+    const int l = min(q >> 7, 3), n = q - l * 128;
+    const long long i = (l == 0 ? s.boff[0] : (l == 1 ? s.boff[1] : (l == 2 ? s.boff[2] : s.boff[3]))) + n;
+    const float g = bgrad[q];
+    grads[i] = g;
+    if (ad.lr > 0.f) adam_step(ad, g, w + i, m + i, v + i);
+}
+
 int grid1(long long n) { return (int)std::min<long long>((n + 255) / 256, 148LL * 8); }
 
 }  // namespace
@@ -273,8 +933,23 @@ struct edus_mlp {
     float* dz = nullptr;
     __nv_bfloat16* dzb = nullptr;
     float* loss = nullptr;
-    int* status = nullptr;  // set when a GEMM's bounded wait for its tensor-core MMAs ran out
+    int* status = nullptr;  // the word after loss: set when a bounded wait in a kernel ran out
+    struct Report {
+        float loss;
+        int status;
+    }* report = nullptr;    // pinned: loss and status of a step, read back in one copy
     cudaStream_t stream = nullptr;
+    // hidden width 128: weight blocks, and per 128-row block the operands of the weight gradients
+    bool blocks = false;
+    MlpShape shape{};
+    __nv_bfloat16* wp = nullptr;
+    int cap_rb = 0;               // row blocks the buffers below hold
+    __nv_bfloat16* actb = nullptr;
+    __nv_bfloat16* dzblk = nullptr;
+    float* dzf = nullptr;
+    float* bgrad = nullptr;
+    float* lossp = nullptr;
+    float* dw = nullptr;          // [tiles][in 128][out 128] weight gradients
 };
 
 namespace {
@@ -292,14 +967,71 @@ int mfail(edus_mlp* m, int code, const std::string& msg) {
         if (e_ != cudaSuccess) return mfail(m, EDUS_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
     } while (0)
 
-// After a synchronisation: report (and clear) a GEMM wait that ran out.
-int mlp_status(edus_mlp* m) {
-    int v = 0;
-    MCU(m, cudaMemcpy(&v, m->status, sizeof(int), cudaMemcpyDeviceToHost));
-    if (v) {
+// Wait for the stream's work; its loss, and a report (cleared) of a wait that ran out.
+int mlp_finish(edus_mlp* m, float* loss_host) {
+    MCU(m, cudaMemcpyAsync(m->report, m->loss, sizeof(*m->report), cudaMemcpyDeviceToHost, m->stream));
+    MCU(m, cudaStreamSynchronize(m->stream));
+    if (loss_host) *loss_host = m->report->loss;
+    if (m->report->status) {
         MCU(m, cudaMemset(m->status, 0, sizeof(int)));
         return mfail(m, EDUS_ERR_TIMEOUT, "a bounded wait for the tensor-core MMAs of a GEMM ran out");
     }
+    return EDUS_OK;
+}
+
+// Buffers of the 128-wide path for B rows.
+int ensure_blocks(edus_mlp* m, int B) {
+    const int nrb = (B + 127) / 128;
+    if (nrb <= m->cap_rb) return EDUS_OK;
+    const int KT = m->shape.KT, NT = m->shape.NT;
+    MCU(m, cudaStreamSynchronize(m->stream));
+    for (void* p : {(void*)m->actb, (void*)m->dzblk, (void*)m->dzf, (void*)m->lossp}) cudaFree(p);
+    m->actb = m->dzblk = nullptr;
+    m->dzf = m->lossp = nullptr;
+    m->cap_rb = 0;
+    MCU(m, cudaMalloc((void**)&m->actb, (size_t)nrb * (KT + 3) * kBlkBytes));
+    MCU(m, cudaMalloc((void**)&m->dzblk, (size_t)nrb * (3 + NT) * kBlkBytes));
+    MCU(m, cudaMalloc((void**)&m->dzf, (size_t)nrb * (3 + NT) * kBlk * sizeof(float)));
+    MCU(m, cudaMalloc((void**)&m->lossp, (size_t)nrb * sizeof(float)));
+    if (!m->dw) MCU(m, cudaMalloc((void**)&m->dw, (size_t)(KT + 2 + NT) * kBlk * sizeof(float)));
+    if (!m->bgrad) MCU(m, cudaMalloc((void**)&m->bgrad, (size_t)(3 + NT) * 128 * sizeof(float)));
+    m->cap_rb = nrb;
+    return EDUS_OK;
+}
+
+MlpRowsArgs rows_args(edus_mlp* m, int B, const float* x, const float* t, float* y) {
+    MlpRowsArgs a{};
+    a.B = B;
+    a.n_in = m->shape.n_in;
+    a.n_out = m->shape.n_out;
+    a.KT = m->shape.KT;
+    a.NT = m->shape.NT;
+    a.x = x;
+    a.t = t;
+    a.y = y;
+    a.wp = m->wp;
+    for (int l = 0; l < kLayers; ++l) a.bias[l] = m->params + m->boff[l];
+    a.act = m->actb;
+    a.dz = m->dzblk;
+    a.dzf = m->dzf;
+    a.lossp = m->lossp;
+    a.scale = 1.f / (float)((long long)B * a.n_out);
+    a.status = m->status;
+    return a;
+}
+
+// Loss and gradients of the batch and, with lr > 0, an Adam step.
+int blocks_backward(edus_mlp* m, int B, const float* x, const float* t, float lr, float c1, float c2) {
+    int rc;
+    if ((rc = ensure_blocks(m, B))) return rc;
+    const int nrb = (B + 127) / 128, tiles = m->shape.KT + 2 + m->shape.NT;
+    mlp_rows_kernel<true><<<nrb, 512, kRowsSmem, m->stream>>>(rows_args(m, B, x, t, nullptr));
+    mlp_dw_kernel<<<dim3(tiles + 3 + m->shape.NT, 4), 128, kDwSmem, m->stream>>>(
+        m->actb, m->dzblk, m->dzf, m->shape.KT, m->shape.NT, nrb, B, m->dw, m->bgrad, m->status);
+    mlp_update_kernel<<<8 * tiles + (384 + m->shape.n_out + 255) / 256 + 1, 256, 0, m->stream>>>(
+        m->shape, m->dw, m->bgrad, m->lossp, nrb, m->grads, m->params, m->wp, m->m, m->v, m->loss,
+        AdamArgs{lr, 0.9f, 0.999f, 1e-8f, c1, c2});
+    MCU(m, cudaGetLastError());
     return EDUS_OK;
 }
 
@@ -394,18 +1126,40 @@ int edus_mlp_create(int n_in, int n_hidden, int n_out, unsigned long long seed, 
         off += m->dims[l + 1];
     }
     m->nparams = off;
-    if (cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking) != cudaSuccess ||
+    m->blocks = n_hidden == 128;
+    if (m->blocks) {
+        m->shape.n_in = n_in;
+        m->shape.n_out = n_out;
+        m->shape.KT = (n_in + 127) / 128;
+        m->shape.NT = (n_out + 127) / 128;
+        m->shape.nparams = off;
+        for (int l = 0; l < kLayers; ++l) {
+            m->shape.woff[l] = m->woff[l];
+            m->shape.boff[l] = m->boff[l];
+        }
+        const size_t wb = (size_t)(m->shape.KT + 2 + m->shape.NT) * kBlkBytes;
+        if (cudaMalloc((void**)&m->wp, wb) != cudaSuccess || cudaMemset(m->wp, 0, wb) != cudaSuccess ||
+            cudaFuncSetAttribute(mlp_rows_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowsSmem) != cudaSuccess ||
+            cudaFuncSetAttribute(mlp_rows_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowsSmem) != cudaSuccess ||
+            cudaFuncSetAttribute(mlp_dw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDwSmem) != cudaSuccess) {
+            edus_mlp_destroy(m);
+            return mfail(nullptr, EDUS_ERR_NOMEM, "MLP weight block set-up failed");
+        }
+    }
+    // a blocking stream: ordered after the legacy stream, where callers prepare their batches
+    if (cudaStreamCreate(&m->stream) != cudaSuccess ||
         cudaMalloc((void**)&m->params, off * sizeof(float)) != cudaSuccess ||
         cudaMalloc((void**)&m->grads, off * sizeof(float)) != cudaSuccess ||
         cudaMalloc((void**)&m->m, off * sizeof(float)) != cudaSuccess ||
         cudaMalloc((void**)&m->v, off * sizeof(float)) != cudaSuccess ||
         cudaMalloc((void**)&m->wbf, off * sizeof(__nv_bfloat16)) != cudaSuccess ||
-        cudaMalloc((void**)&m->loss, sizeof(float)) != cudaSuccess ||
-        cudaMalloc((void**)&m->status, sizeof(int)) != cudaSuccess ||
-        cudaMemset(m->status, 0, sizeof(int)) != cudaSuccess) {
+        cudaMalloc((void**)&m->loss, sizeof(*m->report)) != cudaSuccess ||
+        cudaMallocHost((void**)&m->report, sizeof(*m->report)) != cudaSuccess ||
+        cudaMemset(m->loss, 0, sizeof(*m->report)) != cudaSuccess) {
         edus_mlp_destroy(m);
         return mfail(nullptr, EDUS_ERR_NOMEM, "MLP device allocation failed");
     }
+    m->status = (int*)(m->loss + 1);
     // uniform initialisation scaled by the fan-in (seeded LCG), zero biases
     std::vector<float> p(off, 0.f);
     unsigned long long s = seed * 6364136223846793005ULL + 1442695040888963407ULL;
@@ -436,7 +1190,9 @@ int edus_mlp_destroy(edus_mlp* m) {
     cudaFree(m->v);
     cudaFree(m->wbf);
     cudaFree(m->loss);
-    cudaFree(m->status);
+    if (m->report) cudaFreeHost(m->report);
+    for (void* p : {(void*)m->wp, (void*)m->actb, (void*)m->dzblk, (void*)m->dzf, (void*)m->bgrad, (void*)m->lossp, (void*)m->dw})
+        cudaFree(p);
     for (int l = 0; l < kLayers; ++l) {
         cudaFree(m->z[l]);
         cudaFree(m->a[l]);
@@ -458,7 +1214,8 @@ int edus_mlp_set_params(edus_mlp* m, const float* host) {
     if (!m || !host) return EDUS_ERR_ARG;
     MCU(m, cudaSetDevice(m->device));
     MCU(m, cudaMemcpyAsync(m->params, host, m->nparams * sizeof(float), cudaMemcpyHostToDevice, m->stream));
-    to_bf16_kernel<<<grid1(m->nparams), 256, 0, m->stream>>>(m->params, m->wbf, m->nparams);
+    if (m->blocks) mlp_pack_kernel<<<grid1(m->nparams), 256, 0, m->stream>>>(m->shape, m->params, m->wp);
+    else to_bf16_kernel<<<grid1(m->nparams), 256, 0, m->stream>>>(m->params, m->wbf, m->nparams);
     MCU(m, cudaMemsetAsync(m->m, 0, m->nparams * sizeof(float), m->stream));
     MCU(m, cudaMemsetAsync(m->v, 0, m->nparams * sizeof(float), m->stream));
     m->step = 0;
@@ -478,13 +1235,16 @@ int edus_mlp_forward(edus_mlp* m, int batch, const float* x, float* y) {
     if (!m || !x || !y || batch < 1) return EDUS_ERR_ARG;
     MCU(m, cudaSetDevice(m->device));
     int rc;
-    if ((rc = ensure_cap(m, batch))) return rc;
-    forward(m, batch, x);
-    MCU(m, cudaMemcpyAsync(y, m->z[kLayers - 1], (size_t)batch * m->dims[kLayers] * sizeof(float),
-                           cudaMemcpyDeviceToDevice, m->stream));
+    if (m->blocks) {
+        mlp_rows_kernel<false><<<(batch + 127) / 128, 512, kRowsSmem, m->stream>>>(rows_args(m, batch, x, nullptr, y));
+    } else {
+        if ((rc = ensure_cap(m, batch))) return rc;
+        forward(m, batch, x);
+        MCU(m, cudaMemcpyAsync(y, m->z[kLayers - 1], (size_t)batch * m->dims[kLayers] * sizeof(float),
+                               cudaMemcpyDeviceToDevice, m->stream));
+    }
     MCU(m, cudaGetLastError());
-    MCU(m, cudaStreamSynchronize(m->stream));
-    return mlp_status(m);
+    return mlp_finish(m, nullptr);
 }
 
 int edus_mlp_gradients(edus_mlp* m, int batch, const float* x, const float* target, float* grads_host,
@@ -492,36 +1252,37 @@ int edus_mlp_gradients(edus_mlp* m, int batch, const float* x, const float* targ
     if (!m || !x || !target || batch < 1) return EDUS_ERR_ARG;
     MCU(m, cudaSetDevice(m->device));
     int rc;
-    if ((rc = ensure_cap(m, batch))) return rc;
-    forward(m, batch, x);
-    backward(m, batch, target);
+    if (m->blocks) {
+        if ((rc = blocks_backward(m, batch, x, target, 0.f, 1.f, 1.f))) return rc;
+    } else {
+        if ((rc = ensure_cap(m, batch))) return rc;
+        forward(m, batch, x);
+        backward(m, batch, target);
+    }
     MCU(m, cudaGetLastError());
     if (grads_host)
         MCU(m, cudaMemcpyAsync(grads_host, m->grads, m->nparams * sizeof(float), cudaMemcpyDeviceToHost, m->stream));
-    if (loss_host) MCU(m, cudaMemcpyAsync(loss_host, m->loss, sizeof(float), cudaMemcpyDeviceToHost, m->stream));
-    MCU(m, cudaStreamSynchronize(m->stream));
-    return mlp_status(m);
+    return mlp_finish(m, loss_host);
 }
 
 int edus_mlp_train_step(edus_mlp* m, int batch, const float* x, const float* target, float lr, float* loss_host) {
     if (!m || !x || !target || batch < 1 || !(lr > 0.f)) return EDUS_ERR_ARG;
     MCU(m, cudaSetDevice(m->device));
     int rc;
-    if ((rc = ensure_cap(m, batch))) return rc;
-    forward(m, batch, x);
-    backward(m, batch, target);
+    if ((rc = m->blocks ? ensure_blocks(m, batch) : ensure_cap(m, batch))) return rc;
     m->step++;
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = 1.f - std::pow(b1, (float)m->step), c2 = 1.f - std::pow(b2, (float)m->step);
-    adam_kernel<<<grid1(m->nparams), 256, 0, m->stream>>>(m->params, m->wbf, m->grads, m->m, m->v, m->nparams, lr, b1,
-                                                          b2, 1e-8f, c1, c2);
-    MCU(m, cudaGetLastError());
-    if (loss_host) {
-        MCU(m, cudaMemcpyAsync(loss_host, m->loss, sizeof(float), cudaMemcpyDeviceToHost, m->stream));
-        MCU(m, cudaStreamSynchronize(m->stream));
-        return mlp_status(m);
+    if (m->blocks) {
+        if ((rc = blocks_backward(m, batch, x, target, lr, c1, c2))) return rc;
+    } else {
+        forward(m, batch, x);
+        backward(m, batch, target);
+        adam_kernel<<<grid1(m->nparams), 256, 0, m->stream>>>(m->params, m->wbf, m->grads, m->m, m->v, m->nparams, lr,
+                                                              b1, b2, 1e-8f, c1, c2);
     }
-    return EDUS_OK;
+    MCU(m, cudaGetLastError());
+    return loss_host ? mlp_finish(m, loss_host) : EDUS_OK;
 }
 
 }  // extern "C"
