@@ -305,19 +305,6 @@ __device__ __forceinline__ void mma_k16(unsigned tmem, unsigned long long da, un
 }
 constexpr unsigned kTransA = 1u << 15, kTransB = 1u << 16;
 
-// acc[128][128] (+)= A W^T or A W over a block's K of 128 (8 MMAs of K = 16), by
-// one thread.  A: an activation block (ACT) or a gradient block, K along its
-// columns; W: a weight block, K along its columns (forward) or rows (backward).
-template <bool ACT, bool FORWARD>
-__device__ __forceinline__ void rows_mma(const __nv_bfloat16* A, const __nv_bfloat16* W, unsigned tmem, bool accumulate) {
-#pragma unroll
-    for (int st = 0; st < 8; ++st) {
-        const unsigned long long da = ACT ? op_desc(A + (st >> 1) * kGrp + (st & 1) * 128, 128, 512)
-                                          : op_desc(A + st * 128, 128, 2048);
-        const unsigned long long db = FORWARD ? op_desc(W + st * 128, 128, 2048) : op_desc(W + st * 2048, 2048, 128);
-        mma_k16(tmem, da, db, kUmmaIdesc | (FORWARD ? 0u : kTransB), accumulate || st > 0);
-    }
-}
 // acc[out 128][in 32] (+)= dz^T act over 128 batch rows: both operands MN-major
 __device__ __forceinline__ void dw_mma(const __nv_bfloat16* dz, const __nv_bfloat16* act, unsigned tmem, bool accumulate) {
     constexpr unsigned idesc =
@@ -343,14 +330,6 @@ __device__ __forceinline__ void blk_load(void* dst, const void* src, unsigned lo
                  "l"(reinterpret_cast<unsigned long long>(src)), "r"(bytes), "r"(smem_addr(bar))
                  : "memory");
 }
-// 32 KB block shared -> global, one bulk group of the issuing thread
-__device__ __forceinline__ void blk_store(void* dst, const void* src) {
-    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n" ::"l"(
-                     reinterpret_cast<unsigned long long>(dst)),
-                 "r"(smem_addr(src)), "r"(kBlkBytes)
-                 : "memory");
-    asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
-}
 __device__ __forceinline__ void tmem_ld16(float* v, unsigned addr) {
     unsigned u[16];
     asm volatile(
@@ -363,30 +342,14 @@ __device__ __forceinline__ void tmem_ld16(float* v, unsigned addr) {
 #pragma unroll
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(u[i]);
 }
-// 16 consecutive columns of row r of an activation (ACT) or gradient block, rounded to BF16
-template <bool ACT>
-__device__ __forceinline__ void blk_put16(__nv_bfloat16* blk, int r, int c, const float* v) {
+__device__ __forceinline__ void tmem_ld8(float* v, unsigned addr) {
+    unsigned u[8];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n"
+                 : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7])
+                 : "r"(addr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        __nv_bfloat162 p[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) p[i] = __floats2bfloat162_rn(v[8 * h + 2 * i], v[8 * h + 2 * i + 1]);
-        *reinterpret_cast<uint4*>(blk + (ACT ? act_off(r, c + 8 * h) : blk_off(r, c + 8 * h))) = *reinterpret_cast<uint4*>(p);
-    }
-}
-// v[i] of lane j <-> v[j] of lane i over the warp
-__device__ __forceinline__ void warp_transpose32(float* v, int lane) {
-#pragma unroll
-    for (int s = 16; s >= 1; s >>= 1) {
-        const bool up = lane & s;
-#pragma unroll
-        for (int i = 0; i < 32; ++i) {
-            if (i & s) continue;
-            const float got = __shfl_xor_sync(0xffffffffu, up ? v[i] : v[i + s], s);
-            if (up) v[i] = got;
-            else v[i + s] = got;
-        }
-    }
+    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(u[i]);
 }
 
 struct MlpRowsArgs {
@@ -399,53 +362,85 @@ struct MlpRowsArgs {
     __nv_bfloat16* act;        // [row block][KT + 3]: x blocks, a1, a2, a3 (TRAIN)
     __nv_bfloat16* dz;         // [row block][3 + NT]: dz of layers 0, 1, 2 and of the output blocks (TRAIN)
     float* dzf;                // [row block][3 + NT][4 column groups][128][32]: dz in FP32 (TRAIN)
-    float* lossp;              // [row block] (TRAIN)
+    float* lossp;              // [row block][4] (TRAIN)
     float scale;               // 1 / (B n_out)
     int* status;
 };
 
-// 128 batch rows through the network and, with TRAIN, back.  16 warps; warp w
-// reads tensor-memory lanes 32 (w & 3) .. + 31 (its rows) and the 32 columns from
-// 32 (w >> 2).  Tensor-memory columns: the pre-activations of the three hidden
-// layers at 0, 128, 256, the output block at 384; backward, the gradient of a
-// layer's activations takes the columns of the layer above it.  Every wait is
-// bounded; one that runs out sets *status and ends the CTA.
+constexpr int kTeam = 4;  // CTAs of a row block, a column group each
+
+__device__ __forceinline__ unsigned peer_addr(const void* p, int rank) {
+    unsigned r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(r) : "r"(smem_addr(p)), "r"(rank));
+    return r;
+}
+// every thread of the team, with what each wrote to shared memory (its own and
+// the peers') before it
+__device__ __forceinline__ void team_sync() {
+    asm volatile("fence.proxy.async.shared::cluster;\n" ::: "memory");
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cluster;\n" ::: "memory");
+}
+
+// 128 batch rows through the network and, with TRAIN, back, by a cluster of four
+// CTAs.  CTA j computes columns 32 j .. 32 j + 31 of every 128-wide layer block: its
+// share of the products (N = 32), of GELU and its derivative (erff and expf, the
+// largest part of the time: one CTA a row block, 4096 rows on 32 SMs, took 59 us;
+// four, 26 us) and of the loads and stores.  It writes its columns of an
+// activation or gradient block into all four CTAs' shared memory, so each holds
+// the whole block as the operand of its next product; one cluster barrier a
+// product orders this.  Buffers rotate: when a CTA writes block i it has passed
+// the barrier of block i - 1, so every CTA's product of block i - 2 is done and the
+// buffer of block i - 3 is free.
+//
+// 16 warps; a thread owns one row (32 (warp & 3) + lane, its tensor-memory lane)
+// and 8 columns of the group, 32 bytes of each FP32 row it reads or writes.
+// Tensor-memory columns: the pre-activations of the hidden layers at 0, 32, 64,
+// the output block at 96; backward, the gradient of a layer's activations takes
+// the columns of the layer above it.  Every wait is bounded; one that runs out
+// sets *status and tells the team (`failed`, by the parity of the next barrier,
+// so that all four leave at the same one).
 template <bool TRAIN>
-__global__ void __launch_bounds__(512, 1) mlp_rows_kernel(MlpRowsArgs a) {
+__global__ void __cluster_dims__(kTeam, 1, 1) __launch_bounds__(512, 1) mlp_rows_kernel(MlpRowsArgs a) {
     extern __shared__ unsigned char mraw[];
     __shared__ __align__(8) unsigned long long full[kRing], mma_bar, rel_bar;
     __shared__ unsigned tmem_slot;
-    __shared__ int failed;
+    __shared__ int failed[2];
     __shared__ float red[16];
     __nv_bfloat16* act = (__nv_bfloat16*)(((unsigned long long)mraw + 1023) & ~1023ull);
     __nv_bfloat16* ring = act + kActs * kBlk;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int row = (warp & 3) * 32 + lane, col0 = (warp >> 2) * 32;
-    const int grow = blockIdx.x * 128 + row;
+    const int rank = blockIdx.x & (kTeam - 1), rb = blockIdx.x / kTeam;
+    const int row = (warp & 3) * 32 + lane, sub = (warp >> 2) * 8, col0 = rank * 32 + sub;
+    const long long grow = (long long)rb * 128 + row;
     const bool live = grow < a.B;
     const int KT = a.KT, NT = a.NT;
     const int nqf = KT + 2 + NT, nq = TRAIN ? nqf + NT + 2 : nqf;
+    constexpr unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((32u >> 3) << 17) | ((unsigned)(UM >> 4) << 24);
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_addr(&tmem_slot)),
-                     "r"(512)
+                     "r"(128)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
     }
-    // weight block of product q (forward layers, then backward from the output)
-    auto wblock = [&](int q) {
-        if (q < nqf) return q;
-        const int p = q - nqf;
-        return p < NT ? KT + 2 + p : (p == NT ? KT + 1 : KT);
-    };
     int issued = 0;  // thread 0: weight blocks requested
+    // weight block of product q (forward layers, then backward from the output);
+    // forward this CTA needs the block's 32 output rows only
     auto prefetch = [&](int q) {
-        if (q < nq) {
-            blk_load(ring + (q % kRing) * kBlk, a.wp + (size_t)wblock(q) * kBlk, &full[q % kRing]);
-            issued = q + 1;
+        if (q >= nq) return;
+        __nv_bfloat16* dst = ring + (q % kRing) * kBlk;
+        if (q < nqf) {
+            blk_load(dst + rank * 4096, a.wp + (size_t)q * kBlk + rank * 4096, &full[q % kRing], kBlkBytes / kTeam);
+        } else {
+            const int p = q - nqf;
+            blk_load(dst, a.wp + (size_t)(p < NT ? KT + 2 + p : (p == NT ? KT + 1 : KT)) * kBlk, &full[q % kRing]);
         }
+        issued = q + 1;
     };
     if (tid == 0) {
-        failed = 0;
+        failed[0] = failed[1] = 0;
         for (int i = 0; i < kRing; ++i) bar_init1(&full[i]);
         bar_init1(&mma_bar);
         bar_init1(&rel_bar);
@@ -453,218 +448,215 @@ __global__ void __launch_bounds__(512, 1) mlp_rows_kernel(MlpRowsArgs a) {
         for (int q = 0; q < kRing; ++q) prefetch(q);
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-    __syncthreads();
+    team_sync();  // the peers' shared memory may be written from here on
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     const unsigned tmem = tmem_slot;
-    const unsigned lanes = tmem + ((unsigned)((warp & 3) * 32) << 16);
+    const unsigned lanes = tmem + ((unsigned)((warp & 3) * 32) << 16) + sub;
 
-    // product q: A block (written by this CTA) times the weight block; the
-    // A block also goes to `keep` in global memory for the weight gradients
-    auto product = [&](int q, const __nv_bfloat16* A, bool forward, unsigned col, bool accumulate, __nv_bfloat16* keep) {
-        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+    int nsync = 0;  // team barriers passed in product()
+    auto tell_failed = [&]() {
+        for (int r = 0; r < kTeam; ++r)
+            asm volatile("st.shared::cluster.u32 [%0], %1;\n" ::"r"(peer_addr(&failed[(nsync + 1) & 1], r)), "r"(1) : "memory");
+    };
+    // 8 columns of this thread's row, rounded to BF16, into the block's buffer of all four CTAs
+    auto put8 = [&](int buf, bool activation, const float* v) {
+        __nv_bfloat162 p[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) p[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+        const uint4 u = *reinterpret_cast<uint4*>(p);
+        const __nv_bfloat16* d = act + buf * kBlk + (activation ? act_off(row, col0) : blk_off(row, col0));
+#pragma unroll
+        for (int r = 0; r < kTeam; ++r)
+            asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};\n" ::"r"(peer_addr(d, r)), "r"(u.x), "r"(u.y),
+                         "r"(u.z), "r"(u.w)
+                         : "memory");
+    };
+    // this thread's 8 FP32 of a dz block, for the bias gradients
+    auto put_dzf = [&](int slot, const float* v) {
+        float* d = a.dzf + ((((size_t)rb * (3 + NT) + slot) * 4 + rank) * 128 + row) * 32 + sub;
+        *reinterpret_cast<float4*>(d) = make_float4(v[0], v[1], v[2], v[3]);
+        *reinterpret_cast<float4*>(d + 4) = make_float4(v[4], v[5], v[6], v[7]);
+    };
+    // the team's barrier after a block is written; false: leave (all four CTAs do)
+    auto block_ready = [&]() {
         asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
         // stores older than the last one have left their buffers
         if (TRAIN && tid == 0) asm volatile("cp.async.bulk.wait_group.read 1;\n" ::: "memory");
-        __syncthreads();
+        team_sync();
+        ++nsync;
+        return *(volatile int*)&failed[nsync & 1] == 0;
+    };
+    // a quarter of a block in shared memory to global memory: an activation
+    // block's column group, or a gradient block's 32 rows (8 KB either way)
+    auto store_share = [&](__nv_bfloat16* dst, int buf) {
+        const __nv_bfloat16* src = act + buf * kBlk + rank * (kBlk / kTeam);
+        asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n" ::"l"(
+                         reinterpret_cast<unsigned long long>(dst + rank * (kBlk / kTeam))),
+                     "r"(smem_addr(src)), "r"(kBlkBytes / kTeam)
+                     : "memory");
+        asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
+    };
+    // product q: the block in buffer `buf` times the weight block, into tensor-memory column `col`
+    auto product = [&](int q, int buf, bool forward, unsigned col, bool accumulate) {
         if (tid == 0) {
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            if (!mbar_wait_parity(&full[q % kRing], (unsigned)((q / kRing) & 1), kMlpPolls)) failed = 1;
+            if (!mbar_wait_parity(&full[q % kRing], (unsigned)((q / kRing) & 1), kMlpPolls)) tell_failed();
+            const __nv_bfloat16* A = act + buf * kBlk;
             const __nv_bfloat16* W = ring + (q % kRing) * kBlk;
-            if (forward) rows_mma<true, true>(A, W, tmem + col, accumulate);
-            else rows_mma<false, false>(A, W, tmem + col, accumulate);
+#pragma unroll
+            for (int st = 0; st < 8; ++st) {  // K = 16 each
+                if (forward)
+                    mma_k16(tmem + col, op_desc(A + (st >> 1) * kGrp + (st & 1) * 128, 128, 512),
+                            op_desc(W + rank * 4096 + st * 128, 128, 2048), idesc, accumulate || st > 0);
+                else
+                    mma_k16(tmem + col, op_desc(A + st * 128, 128, 2048), op_desc(W + rank * 256 + st * 2048, 2048, 128),
+                            idesc | kTransB, accumulate || st > 0);
+            }
             mma_commit(&mma_bar);
-            if (TRAIN && keep) blk_store(keep, A);
         }
     };
-    // product q is done (all threads agree); its weight block's slot is refilled
+    // product q is done; its weight block's slot is refilled
     auto finished = [&](int q) {
         const bool ok = mbar_wait_parity(&mma_bar, (unsigned)(q & 1), kMlpPolls);
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-        if (__syncthreads_or(!ok || failed)) return false;
+        if (!ok) tell_failed();
+        __syncthreads();
         if (tid == 0) prefetch(q + kRing);
-        return true;
+        __syncwarp();
     };
-    __nv_bfloat16* keep_act = TRAIN ? a.act + (size_t)blockIdx.x * (KT + 3) * kBlk : nullptr;
-    __nv_bfloat16* keep_dz = TRAIN ? a.dz + (size_t)blockIdx.x * (3 + NT) * kBlk : nullptr;
+    __nv_bfloat16* keep_act = TRAIN ? a.act + (size_t)rb * (KT + 3) * kBlk : nullptr;
+    __nv_bfloat16* keep_dz = TRAIN ? a.dz + (size_t)rb * (3 + NT) * kBlk : nullptr;
+    auto load8 = [&](const float* src, int width, int c, float* v) {  // 8 of this thread's row; zeros past the ends
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = (live && c + i < width) ? __ldg(src + grow * width + c + i) : 0.f;
+    };
+
+    // activation block i sits in buffer i % kActs
+    int q = 0, i = 0;
     bool ok = true;
-    int nblk = 0;  // activation blocks written so far: block i sits in buffer i % kActs
-    auto buffer = [&](int i) { return act + (i % kActs) * kBlk; };
-
-    // 128 rows x 128 input features, FP32 to BF16 (a warp's 32 loads a lane are
-    // in flight together); rows and features past the ends are zero
-    auto load_x = [&](int kt, __nv_bfloat16* dst) {
-        const int r0 = warp * 8;
-        float v[8][4];
-#pragma unroll
-        for (int r = 0; r < 8; ++r) {
-            const long long gr = (long long)blockIdx.x * 128 + r0 + r;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int c = kt * 128 + lane + 32 * j;
-                v[r][j] = (gr < a.B && c < a.n_in) ? __ldg(a.x + gr * a.n_in + c) : 0.f;
-            }
-        }
-#pragma unroll
-        for (int r = 0; r < 8; ++r)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) dst[act_off(r0 + r, lane + 32 * j)] = __float2bfloat16(v[r][j]);
-    };
-    // the warp's 32 x 32 of dz in FP32, for the bias gradients (v is spent)
-    auto put_dzf = [&](float* v, int slot) {
-        warp_transpose32(v, lane);
-        float* d = a.dzf + ((((size_t)blockIdx.x * (3 + NT) + slot) * 4 + (warp >> 2)) * 128 + (warp & 3) * 32) * 32 + lane;
-#pragma unroll
-        for (int i = 0; i < 32; ++i) d[i * 32] = v[i];
-    };
-
-    int q = 0;
-    load_x(0, buffer(nblk));
-    for (int kt = 0; ok && kt < KT; ++kt, ++q) {
-        product(q, buffer(nblk), true, 0, kt > 0, TRAIN ? keep_act + (size_t)kt * kBlk : nullptr);
-        ++nblk;
-        if (kt + 1 < KT) load_x(kt + 1, buffer(nblk));
-        ok = finished(q);
+    float v[8], z[8];
+    load8(a.x, a.n_in, col0, v);
+    for (int kt = 0; ok && kt < KT; ++kt, ++i, ++q) {
+        put8(i % kActs, true, v);
+        if (kt + 1 < KT) load8(a.x, a.n_in, (kt + 1) * 128 + col0, v);
+        if (!(ok = block_ready())) break;
+        product(q, i % kActs, true, 0, kt > 0);
+        if (TRAIN && tid == 0) store_share(keep_act + (size_t)kt * kBlk, i % kActs);
+        finished(q);
     }
-    for (int l = 0; ok && l < 3; ++l) {
-        __nv_bfloat16* dst = buffer(nblk++);
-#pragma unroll 1
-        for (int c0 = col0; c0 < col0 + 32; c0 += 16) {
-            float v[16];
-            tmem_ld16(v, lanes + l * 128 + c0);
+    for (int l = 0; ok && l < 3; ++l, ++i) {
+        tmem_ld8(v, lanes + l * 32);
 #pragma unroll
-            for (int i = 0; i < 16; ++i) v[i] = gelu(v[i] + __ldg(&a.bias[l][c0 + i]));
-            blk_put16<true>(dst, row, c0, v);
-        }
+        for (int j = 0; j < 8; ++j) v[j] = gelu(v[j] + __ldg(&a.bias[l][col0 + j]));
+        put8(i % kActs, true, v);
+        if (!(ok = block_ready())) break;
+        if (TRAIN && tid == 0) store_share(keep_act + (size_t)(KT + l) * kBlk, i % kActs);
         if (l < 2) {
-            product(q, dst, true, (l + 1) * 128, false, TRAIN ? keep_act + (size_t)(KT + l) * kBlk : nullptr);
-            ok = finished(q++);
+            product(q, i % kActs, true, (l + 1) * 32, false);
+            finished(q++);
         }
     }
-    const __nv_bfloat16* a3 = buffer(nblk - 1);
-    const int b3 = nblk - 1;
+    const int b3 = i - 1;  // a3's block
     float loss = 0.f;
     for (int nt = 0; ok && nt < NT; ++nt) {
-        // the warp's 32 x 32 targets, row by row (coalesced), before the product's wait
         const int col = nt * 128 + col0;
-        const long long wrow = (long long)blockIdx.x * 128 + (warp & 3) * 32;
-        float tv[32];
-        if (TRAIN) {
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-                tv[i] = (wrow + i < a.B && col + lane < a.n_out) ? __ldg(a.t + (wrow + i) * a.n_out + col + lane) : 0.f;
-        }
-        product(q, a3, true, 384, false, (TRAIN && nt == 0) ? keep_act + (size_t)(KT + 2) * kBlk : nullptr);
-        ok = finished(q++);
-        if (!ok) break;
-        // output blocks take turns in the two buffers that a3 leaves; an earlier
-        // block's store has left its buffer (product() waited for it)
-        __nv_bfloat16* dst = buffer(b3 + 1 + (nt & 1));
-        float v[32];
-        tmem_ld16(v, lanes + 384 + col0);
-        tmem_ld16(v + 16, lanes + 384 + col0 + 16);
-        if (TRAIN) {
-            warp_transpose32(tv, lane);
-#pragma unroll
-            for (int i = 0; i < 32; ++i) {
-                const bool on = live && col + i < a.n_out;
-                const float d = on ? v[i] + __ldg(&a.bias[3][col + i]) - tv[i] : 0.f;
-                loss += d * d;
-                v[i] = 2.f * d * a.scale;
-            }
-            blk_put16<false>(dst, row, col0, v);
-            blk_put16<false>(dst, row, col0 + 16, v + 16);
-            put_dzf(v, 3 + nt);
-        } else {
-            warp_transpose32(v, lane);
-            const float bias = col + lane < a.n_out ? __ldg(&a.bias[3][col + lane]) : 0.f;
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-                if (wrow + i < a.B && col + lane < a.n_out) a.y[(wrow + i) * a.n_out + col + lane] = v[i] + bias;
-        }
-        if (TRAIN) {
-            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+        if (TRAIN) load8(a.t, a.n_out, col, z);
+        product(q, b3 % kActs, true, 96, false);
+        finished(q++);
+        tmem_ld8(v, lanes + 96);
+        if (!TRAIN) {
+            // the next product overwrites these columns
+            asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
             __syncthreads();
-            if (tid == 0) {
-                blk_store(keep_dz + (size_t)(3 + nt) * kBlk, dst);
-                // the other buffer is free before the next block is written there
-                asm volatile("cp.async.bulk.wait_group.read 1;\n" ::: "memory");
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                if (live && col + j < a.n_out) a.y[grow * a.n_out + col + j] = v[j] + __ldg(&a.bias[3][col + j]);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const bool on = live && col + j < a.n_out;
+                const float d = on ? v[j] + __ldg(&a.bias[3][col + j]) - z[j] : 0.f;
+                loss += d * d;
+                v[j] = 2.f * d * a.scale;
             }
+            // output blocks take turns in the two buffers that a3 leaves
+            const int buf = (b3 + 1 + (nt & 1)) % kActs;
+            if (nt >= 2) {
+                // the block before last has left its buffer in every CTA
+                if (tid == 0) asm volatile("cp.async.bulk.wait_group.read 1;\n" ::: "memory");
+                team_sync();
+            }
+            put8(buf, false, v);
+            if (!(ok = block_ready())) break;
+            if (tid == 0) store_share(keep_dz + (size_t)(3 + nt) * kBlk, buf);
+            put_dzf(3 + nt, v);
         }
     }
     if (TRAIN) {
-        __syncthreads();
-        if (ok) {
-            // loss of these rows
 #pragma unroll
-            for (int s = 16; s > 0; s >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, s);
-            if (lane == 0) red[warp] = loss;
-            __syncthreads();
-            if (tid == 0) {
-                float s = 0.f;
-                for (int i = 0; i < 16; ++i) s += red[i];
-                a.lossp[blockIdx.x] = s * a.scale;
-            }
+        for (int s = 16; s > 0; s >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, s);
+        if (lane == 0) red[warp] = loss;
+        __syncthreads();
+        if (tid == 0) {
+            float s = 0.f;
+            for (int w = 0; w < 16; ++w) s += red[w];
+            a.lossp[rb * kTeam + rank] = s * a.scale;
         }
-        // gradient of a3: sum over the output blocks of dz_out W^T (columns 384; more
+        // gradient of a3: sum over the output blocks of dz_out W^T (column 96; more
         // than two blocks are read back from global memory)
-        int nrel = 0;
+        if (NT > 2) {
+            if (tid == 0) asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory");  // the blocks are written
+            asm volatile("fence.proxy.async.global;\n" ::: "memory");
+            team_sync();
+            asm volatile("fence.proxy.async.global;\n" ::: "memory");
+        }
         for (int nt = 0; ok && nt < NT; ++nt) {
-            const __nv_bfloat16* A = buffer(b3 + 1 + (nt & 1));
+            const int buf = (b3 + 1 + (nt & 1)) % kActs;
             if (NT > 2) {
                 if (tid == 0) {
-                    asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory");  // the blocks are written
-                    blk_load(act + (size_t)((b3 + 1 + (nt & 1)) % kActs) * kBlk, keep_dz + (size_t)(3 + nt) * kBlk, &rel_bar);
+                    blk_load(act + buf * kBlk, keep_dz + (size_t)(3 + nt) * kBlk, &rel_bar);
+                    if (!mbar_wait_parity(&rel_bar, (unsigned)(nt & 1), kMlpPolls)) tell_failed();
                 }
-                const bool got = mbar_wait_parity(&rel_bar, (unsigned)(nrel & 1), kMlpPolls);
-                ++nrel;
-                if (__syncthreads_or(!got)) {
-                    ok = false;
-                    break;
-                }
-            }
-            product(q, A, false, 384, nt > 0, nullptr);
-            ok = finished(q++);
-        }
-        nblk = b3 + 3;  // the next buffer is a3's, whose products and store are done
-        for (int l = 2; ok && l >= 0; --l) {
-            // dz_l = da * GELU'(z_l): da in columns (l + 1) * 128, z_l in l * 128
-            if (tid == 0) asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");
-            __syncthreads();
-            __nv_bfloat16* dst = buffer(nblk++);
-            float v[32];
-#pragma unroll
-            for (int c0 = 0; c0 < 32; c0 += 16) {
-                float z[16];
-                tmem_ld16(v + c0, lanes + (l + 1) * 128 + col0 + c0);
-                tmem_ld16(z, lanes + l * 128 + col0 + c0);
-#pragma unroll
-                for (int i = 0; i < 16; ++i) v[c0 + i] *= gelu_grad(z[i] + __ldg(&a.bias[l][col0 + c0 + i]));
-                blk_put16<false>(dst, row, col0 + c0, v + c0);
-            }
-            put_dzf(v, l);
-            if (l > 0) {
-                product(q, dst, false, l * 128, false, keep_dz + (size_t)l * kBlk);
-                ok = finished(q++);
-            } else {
-                asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
                 __syncthreads();
-                if (tid == 0) blk_store(keep_dz, dst);
             }
+            product(q, buf, false, 96, nt > 0);
+            finished(q++);
+        }
+        // the next blocks' buffers: a3's, then the output blocks'
+        i = b3 + 3;
+        for (int l = 2; ok && l >= 0; --l, ++i) {
+            // dz_l = da * GELU'(z_l)
+            tmem_ld8(v, lanes + (l + 1) * 32);
+            tmem_ld8(z, lanes + l * 32);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] *= gelu_grad(z[j] + __ldg(&a.bias[l][col0 + j]));
+            if (l == 2) {
+                // every CTA's products and stores of the buffers written from here on are done
+                if (tid == 0) asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");
+                team_sync();
+            }
+            put8(i % kActs, false, v);
+            if (!(ok = block_ready())) break;
+            if (l > 0) product(q, i % kActs, false, l * 32, false);
+            if (tid == 0) store_share(keep_dz + (size_t)l * kBlk, i % kActs);
+            put_dzf(l, v);
+            if (l > 0) finished(q++);
         }
     }
     if (tid == 0) {
         if (!ok) {
             atomicOr(a.status, 1);
             // weight blocks still in flight land before the CTA ends
-            for (int i = issued - 1; i >= 0 && i >= issued - kRing; --i)
-                mbar_wait_parity(&full[i % kRing], (unsigned)((i / kRing) & 1), kMlpPolls);
+            for (int j = issued - 1; j >= 0 && j >= issued - kRing; --j)
+                mbar_wait_parity(&full[j % kRing], (unsigned)((j / kRing) & 1), kMlpPolls);
         }
         asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-    __syncthreads();
+    team_sync();  // no peer writes this CTA's shared memory any more
+    if (tid == 0 && (failed[0] | failed[1])) atomicOr(a.status, 1);
     if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(512) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(128) : "memory");
 }
 
 // Weight gradients: CTA (tile, group) contracts over the whole batch in row
@@ -710,12 +702,12 @@ __global__ void __launch_bounds__(128, 1) mlp_dw_kernel(const __nv_bfloat16* __r
             const float* d = (const float*)(buf + (size_t)(i % kDwStages) * kBiasStage) + lane;
             const int rows = min(128, B - i * 128);
             int r = 0;
-            for (; r + 16 <= rows; r += 16) {
-                float x[16];
+            for (; r + 32 <= rows; r += 32) {
+                float x[32];
 #pragma unroll
-                for (int j = 0; j < 16; ++j) x[j] = d[(r + j) * 32];
+                for (int j = 0; j < 32; ++j) x[j] = d[(r + j) * 32];
 #pragma unroll
-                for (int j = 0; j < 16; ++j) sum += x[j];
+                for (int j = 0; j < 32; ++j) sum += x[j];
             }
             for (; r < rows; ++r) sum += d[r * 32];
             __syncwarp();
@@ -856,7 +848,7 @@ __device__ __forceinline__ float adam_step(const AdamArgs& ad, float g, float* w
 }
 __global__ void __launch_bounds__(256) mlp_update_kernel(MlpShape s, const float* __restrict__ dw,
                                                          const float* __restrict__ bgrad,
-                                                         const float* __restrict__ lossp, int nrb,
+                                                         const float* __restrict__ lossp, int nloss,
                                                          float* __restrict__ grads, float* __restrict__ w,
                                                          __nv_bfloat16* __restrict__ wp, float* __restrict__ m,
                                                          float* __restrict__ v, float* __restrict__ loss, AdamArgs ad) {
@@ -893,7 +885,7 @@ __global__ void __launch_bounds__(256) mlp_update_kernel(MlpShape s, const float
     if (blockIdx.x == gridDim.x - 1) {
         if (threadIdx.x >= 32) return;
         float t = 0.f;
-        for (int i = threadIdx.x; i < nrb; i += 32) t += lossp[i];
+        for (int i = threadIdx.x; i < nloss; i += 32) t += lossp[i];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
         if (threadIdx.x == 0) *loss = t;
@@ -992,7 +984,7 @@ int ensure_blocks(edus_mlp* m, int B) {
     MCU(m, cudaMalloc((void**)&m->actb, (size_t)nrb * (KT + 3) * kBlkBytes));
     MCU(m, cudaMalloc((void**)&m->dzblk, (size_t)nrb * (3 + NT) * kBlkBytes));
     MCU(m, cudaMalloc((void**)&m->dzf, (size_t)nrb * (3 + NT) * kBlk * sizeof(float)));
-    MCU(m, cudaMalloc((void**)&m->lossp, (size_t)nrb * sizeof(float)));
+    MCU(m, cudaMalloc((void**)&m->lossp, (size_t)nrb * kTeam * sizeof(float)));
     if (!m->dw) MCU(m, cudaMalloc((void**)&m->dw, (size_t)(KT + 2 + NT) * kBlk * sizeof(float)));
     if (!m->bgrad) MCU(m, cudaMalloc((void**)&m->bgrad, (size_t)(3 + NT) * 128 * sizeof(float)));
     m->cap_rb = nrb;
@@ -1025,11 +1017,11 @@ int blocks_backward(edus_mlp* m, int B, const float* x, const float* t, float lr
     int rc;
     if ((rc = ensure_blocks(m, B))) return rc;
     const int nrb = (B + 127) / 128, tiles = m->shape.KT + 2 + m->shape.NT;
-    mlp_rows_kernel<true><<<nrb, 512, kRowsSmem, m->stream>>>(rows_args(m, B, x, t, nullptr));
+    mlp_rows_kernel<true><<<kTeam * nrb, 512, kRowsSmem, m->stream>>>(rows_args(m, B, x, t, nullptr));
     mlp_dw_kernel<<<dim3(tiles + 3 + m->shape.NT, 4), 128, kDwSmem, m->stream>>>(
         m->actb, m->dzblk, m->dzf, m->shape.KT, m->shape.NT, nrb, B, m->dw, m->bgrad, m->status);
     mlp_update_kernel<<<8 * tiles + (384 + m->shape.n_out + 255) / 256 + 1, 256, 0, m->stream>>>(
-        m->shape, m->dw, m->bgrad, m->lossp, nrb, m->grads, m->params, m->wp, m->m, m->v, m->loss,
+        m->shape, m->dw, m->bgrad, m->lossp, kTeam * nrb, m->grads, m->params, m->wp, m->m, m->v, m->loss,
         AdamArgs{lr, 0.9f, 0.999f, 1e-8f, c1, c2});
     MCU(m, cudaGetLastError());
     return EDUS_OK;
@@ -1236,7 +1228,8 @@ int edus_mlp_forward(edus_mlp* m, int batch, const float* x, float* y) {
     MCU(m, cudaSetDevice(m->device));
     int rc;
     if (m->blocks) {
-        mlp_rows_kernel<false><<<(batch + 127) / 128, 512, kRowsSmem, m->stream>>>(rows_args(m, batch, x, nullptr, y));
+        mlp_rows_kernel<false><<<kTeam * ((batch + 127) / 128), 512, kRowsSmem, m->stream>>>(
+            rows_args(m, batch, x, nullptr, y));
     } else {
         if ((rc = ensure_cap(m, batch))) return rc;
         forward(m, batch, x);
