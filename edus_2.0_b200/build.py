@@ -18,8 +18,8 @@ CSRC = os.path.join(PKG, "csrc")
 LIBDIR = os.path.join(PKG, "lib")
 LIB = os.path.join(LIBDIR, "libedus_gpu.so")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-SOURCES = ["edus_gpu.cu", "edus_noalloc.cu", "surrogate.cu"]
-HEADERS = ["comm_ws.cuh", "fft_plane.cuh", "kernels.cuh", "packed_kernels.cuh", "plane3.cuh", "plane_plan.hpp", "split_kernels.cuh", "sweep_kernels.cuh", "tma.cuh"]
+SOURCES = ["edus_gpu.cu", "edus_noalloc.cu", "resident.cu", "surrogate.cu"]
+HEADERS = ["comm_ws.cuh", "fft_plane.cuh", "kernels.cuh", "packed_kernels.cuh", "plane3.cuh", "plane_plan.hpp", "resident.cuh", "split_kernels.cuh", "stage_field.hpp", "sweep_kernels.cuh", "tma.cuh"]
 
 
 def nvcc() -> str:
@@ -42,16 +42,23 @@ def build(force: bool = False, verbose: bool = False) -> str:
     deps.append(os.path.join(ROOT, "include", "edus_gpu.h"))
     if not force and not _stale(LIB, deps):
         return LIB
-    cmd = [nvcc(), *ARCH, "-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-shared",
-           "-o", LIB] + [os.path.join(CSRC, f) for f in SOURCES]
+    flags = [*ARCH, "-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC"]
     if verbose:
-        cmd.insert(-len(SOURCES), "-Xptxas")
-        cmd.insert(-len(SOURCES), "-v")
+        flags += ["-Xptxas", "-v"]
     env = dict(os.environ)
     # the host compiler must be the system gcc (its OpenMP/libstdc++ match the image)
     env.pop("CC", None)
     env.pop("CXX", None)
-    subprocess.run(cmd, check=True, env=env)
+    # the translation units compile side by side
+    objs = [os.path.join(LIBDIR, os.path.splitext(f)[0] + ".o") for f in SOURCES]
+    stale = [(f, o) for f, o in zip(SOURCES, objs) if force or _stale(o, [os.path.join(CSRC, f)] + deps[len(SOURCES):])]
+    procs = [subprocess.Popen([nvcc(), *flags, "-c", os.path.join(CSRC, f), "-o", o], env=env) for f, o in stale]
+    if any([p.wait() for p in procs]):
+        for _, o in stale:
+            if os.path.exists(o):
+                os.remove(o)
+        raise RuntimeError("nvcc failed")
+    subprocess.run([nvcc(), *ARCH, "-Xcompiler", "-fPIC", "-shared", "-o", LIB, *objs], check=True, env=env)
     return LIB
 
 

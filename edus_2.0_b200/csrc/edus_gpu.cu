@@ -19,6 +19,7 @@
 #include "split_kernels.cuh"
 #include "plane3.cuh"
 #include "sweep_kernels.cuh"
+#include "resident.cuh"
 #include <cudaTypedefs.h>
 #include <map>
 #include <mutex>
@@ -67,7 +68,8 @@ struct edus_handle {
     // observables: eigenvectors U_k and velocity operator v_d(k), [P][Nk] each
     double2* obsU = nullptr;
     double2* obsV[3] = {nullptr, nullptr, nullptr};
-    double* obsacc = nullptr;
+    double* obsacc = nullptr;      // sums and the status word, then the CTAs' partial sums and their counter
+    double* obs_host = nullptr;    // pinned
     // a model (H0, xi) per solve (edus_upload_model_solve): [B][P][Nk] each
     bool per_solve = false;
     double2* H0b = nullptr;
@@ -111,6 +113,8 @@ struct edus_handle {
     int nroot_s = 0, nrpos_s = 0;  // persistent plane kernel: root / coordinate entries it stages in shared memory
     int tab_smem = 0;              // their bytes (0: read from global memory)
     int wait_polls = 1 << 22;      // the plane kernel's bulk-load wait limit (edus_set_wait_limit)
+    bool res_ok = false;           // whole calls in one launch (resident.cuh)
+    ResidentGeom res{};
     double2* plane_scratch = nullptr;  // [plane_grid][Nk]: rho(R) between the two inverse transforms
     unsigned long long launches = 0;
     size_t dev_bytes = 0;
@@ -688,6 +692,140 @@ StageArgs base_args(edus_handle* h) {
 
 
 // ---------------------------------------------------------------------------
+// resident steps of small problems (resident.cuh)
+
+ResidentKernel resident_kernel_of(const edus_handle* h) {
+    return resident_kernel(h->d.coulomb != 0, h->d.solver == EDUS_SOLVER_RK, h->plane_cfg.variant == 2);
+}
+
+cudaLaunchConfig_t resident_config(const edus_handle* h, const ResidentGeom& g, cudaLaunchAttribute* attr) {
+    attr->id = cudaLaunchAttributeClusterDimension;
+    attr->val.clusterDim.x = g.CS;
+    attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(g.CS * h->B);
+    c.blockDim = dim3(g.threads);
+    c.dynamicSmemBytes = g.smem;
+    c.stream = h->stream;
+    c.attrs = attr;
+    c.numAttrs = 1;
+    return c;
+}
+
+// Does this handle step by the resident kernel now?  (A profiled handle keeps
+// its launches apart.)
+bool resident_active(const edus_handle* h) {
+    return h->res_ok && !h->profiling && !h->peierls && h->kg_n == 0 && h->nO == 0;
+}
+
+// `cnt` steps in one launch, their field table being in h->field.
+int launch_resident(edus_handle* h, int cnt) {
+    ResidentArgs a{};
+    const StageArgs sa = base_args(h);
+    a.H0 = sa.H0;
+    for (int d = 0; d < 3; ++d) a.xi[d] = sa.xi[d];
+    a.mstride = sa.mstride;
+    a.rho0p = h->rho0p;
+    a.Wp = h->Wp;
+    a.hartree = h->hartree;
+    a.rho0diag = h->rho0diag;
+    a.y = h->y;
+    a.acc = h->acc;  // buffers of the launches per stage, free here
+    a.ham = h->G;
+    a.order = h->d.order;
+    if (h->d.solver == EDUS_SOLVER_AB)
+        for (int q = 0; q < h->d.order; ++q) {
+            a.hist[q] = h->hist[h->index[q]];
+            a.c[q] = h->d.dt * h->beta[q];
+        }
+    a.field = h->field;
+    a.steps = cnt;
+    a.B = h->B;
+    a.roots = h->roots;
+    a.rpos = h->rpos;
+    a.ntab = h->N[0] + h->N[1] + h->N[2];
+    a.S = (long long)h->S;
+    a.Nk = h->Nk;
+    a.nb = h->nb;
+    a.inv_nk = 1.0 / h->Nk;
+    a.dt = h->d.dt;
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t c = resident_config(h, h->res, &attr);
+    CU(h, cudaLaunchKernelEx(&c, resident_kernel_of(h), a, h->res, h->plan));
+    h->launches++;
+    for (int i = 0; i < cnt; ++i) {
+        h->t += h->d.dt;
+        if (h->d.solver == EDUS_SOLVER_AB) {
+            // rotate the ring (DESolver.hpp:212-217)
+            const int ord = h->d.order;
+            const int tmp = h->index[ord - 1];
+            for (int q = ord - 1; q > 0; --q) h->index[q] = h->index[q - 1];
+            h->index[0] = tmp;
+        }
+    }
+    return EDUS_OK;
+}
+
+// Estimated cycles of one stage in the resident kernel, fitted to measured
+// phases: a butterfly round of radix R costs 500 + 100 R, a round of 2 x 2
+// commutator tiles 1500 + 450 nb, an exchange between CTAs 1200 and 1.2 an
+// element, the model Hamiltonian (every other stage) 5000 a round of four
+// elements.
+double resident_cycles(const edus_handle* h, const ResidentGeom& g) {
+    const bool c = h->d.coulomb != 0;
+    const double rows = (double)h->P * g.RC * (h->Nk / h->N[0]), cols = (double)h->N[0] * g.NC;
+    auto rounds = [&](double tasks) { return std::ceil(tasks / g.threads); };
+    double cyc = 400.0 + (c ? 1200.0 : 0.0);
+    for (int d = 0; d < 3; ++d)
+        for (int s = 0; s < h->plan.ax[d].nst; ++s) {
+            const int r = h->plan.ax[d].r[s];
+            const double pts = d == 0 ? cols : rows;
+            cyc += (rounds(pts / r) + rounds(pts * (c ? 2 : 1) / r)) * (500.0 + 100.0 * r);
+        }
+    const int half = (h->nb + 1) / 2;
+    cyc += rounds((double)half * half * rows / h->P) * (1500.0 + 450.0 * h->nb);
+    cyc += 0.5 * rounds(rows / 4) * 5000.0;
+    return cyc + (g.CS > 1 ? 2.0 * (1200.0 + 1.2 * rows) : 0.0);
+}
+
+// Choose the cluster size and decide whether the handle steps this way.
+int resident_setup(edus_handle* h) {
+    const bool c = h->d.coulomb != 0, rk = h->d.solver == EDUS_SOLVER_RK;
+    const int lim = device_smem_optin(h->d.device);
+    const int ntab = h->N[0] + h->N[1] + h->N[2];
+    ResidentKernel k = resident_kernel_of(h);
+    double best = 1e30;
+    for (int cs : {1, 2, 4, 8, 16}) {
+        if (cs > h->N[0]) break;
+        const ResidentGeom g = resident_geometry(h->plan, h->nb, c, rk, cs, ntab, (size_t)lim);
+        if (!g.smem) continue;
+        const double cyc = resident_cycles(h, g);
+        if (cyc < best) {
+            best = cyc;
+            h->res = g;
+        }
+    }
+    if (best > 1e29) return EDUS_OK;
+    int rc;
+    if ((rc = set_smem(h, k, (int)h->res.smem))) return rc;
+    if (h->res.CS > 8) CU(h, cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t cfg = resident_config(h, h->res, &attr);
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, k, &cfg) != cudaSuccess || clusters < 1) {
+        cudaGetLastError();  // the device cannot place such a cluster: the launches per stage remain
+        return EDUS_OK;
+    }
+    // The launches per stage instead: two kernels (four where planes are spread
+    // over many CTAs) of 4.5-5 us each when nothing but latency counts, and ten
+    // array passes over the solves' states at about 2 TB/s.
+    const double waves = std::ceil((double)h->B / clusters);
+    const double launches_us = (h->use3 ? 20.0 : 9.0) + 160.0 * (double)h->S * h->B / 2.0e6;
+    h->res_ok = 1.2 * best * waves / 1900.0 < launches_us;
+    return EDUS_OK;
+}
+
+// ---------------------------------------------------------------------------
 // packed-Hermitian forms: launch helpers
 
 template <typename C, typename IT, bool COUL>
@@ -897,10 +1035,6 @@ int anchor_split(edus_handle* h) {
     return EDUS_OK;
 }
 
-// One CTA per k point: contributions of that k to the Bloch populations
-// Re (U^dagger rho U)_nn, the Wannier populations Re rho_nn and tr(v_d rho),
-// accumulated in acc[0..nb) (Bloch), acc[nb..2nb) (Wannier), acc[2nb..2nb+6)
-// (re, im of d = 0, 1, 2).  Shared memory: rho_k and U_k, [n][m].
 // Peierls gauge, observables (Simulation.cpp:447-449, 593-595): the state
 // that the populations and the velocity see is rho(R) e^{-iA.R} back in k,
 // one plane per CTA: dst = FFT_{+1}(FFT_{-1}(src) e^{-iA.R} / Nk).
@@ -924,50 +1058,137 @@ __global__ void __launch_bounds__(MAXT) peierls_shift_kernel(const double2* __re
     for (int i = threadIdx.x; i < Nk; i += blockDim.x) dst[off + i] = xs[i];
 }
 
-__global__ void observables_kernel(const double2* __restrict__ rho, const double2* __restrict__ U,
-                                   const double2* __restrict__ v0, const double2* __restrict__ v1,
-                                   const double2* __restrict__ v2, int Nk, int nb, double* __restrict__ acc) {
-    extern __shared__ double2 so[];
-    const int k = blockIdx.x, P = nb * nb;
-    double2* R = so;
-    double2* Us = so + P;
-    for (int p = threadIdx.x; p < P; p += blockDim.x) {
-        R[p] = rho[(long long)p * Nk + k];
-        Us[p] = U ? U[(long long)p * Nk + k] : make_double2(0.0, 0.0);
-    }
+// Observables: sums over k of the Bloch populations Re (U^dagger rho U)_nn
+// (values 0 .. nb - 1), the Wannier populations Re rho_nn (nb ..) and tr(v_d rho)
+// (2 nb ..: re, im of d = 0, 1, 2).
+// The CTAs' sums (fixed order: the result does not depend on which finishes
+// last) and the handle's status word into out, by the last CTA: part[cta][nacc].
+__device__ __forceinline__ void observables_finish(const double* mine, int nacc, double* __restrict__ part,
+                                                   double* __restrict__ out, const int* __restrict__ status,
+                                                   unsigned* __restrict__ count) {
+    for (int v = threadIdx.x; v < nacc; v += blockDim.x) part[(size_t)blockIdx.x * nacc + v] = mine[v];
+    __threadfence();
     __syncthreads();
-    for (int n = threadIdx.x; n < nb; n += blockDim.x) {
-        if (U) {
-            double bl = 0.0;
+    if (!__syncthreads_or(threadIdx.x == 0 && atomicAdd(count, 1u) == gridDim.x - 1)) return;
+    __threadfence();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int v = warp; v < nacc; v += blockDim.x >> 5) {
+        double s = 0.0;
+        for (int c = lane; c < (int)gridDim.x; c += 32) s += __ldcg(&part[(size_t)c * nacc + v]);
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == 0) out[v] = s;
+    }
+    if (threadIdx.x == 0) {
+        out[nacc] = (double)*status;
+        *count = 0;
+    }
+}
+
+// Few bands (nb <= 8): a thread per k point, planes read coalesced along k.
+// One CTA per k point with an atomic per value (the general kernel's first form)
+// took 80 us for two bands on 50 x 50, all of it contention on ten words; 7 us here.
+__global__ void __launch_bounds__(128) observables_thread_kernel(
+    const double2* __restrict__ rho, const double2* __restrict__ U, const double2* __restrict__ v0,
+    const double2* __restrict__ v1, const double2* __restrict__ v2, int Nk, int nb, double* __restrict__ part,
+    double* __restrict__ out, const int* __restrict__ status, unsigned* __restrict__ count) {
+    __shared__ double red[4][22], mine[22];
+    const int nacc = 2 * nb + 6, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int k = blockIdx.x * 128 + threadIdx.x;
+    const bool on = k < Nk;
+    auto put = [&](int v, double x) {
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        if (lane == 0) red[warp][v] = x;
+    };
+    for (int n = 0; n < nb; ++n) {
+        double bl = 0.0;
+        if (U && on)
             for (int i = 0; i < nb; ++i) {
                 double2 t = make_double2(0.0, 0.0);
-                for (int j = 0; j < nb; ++j) t = cadd(t, cmul(R[i * nb + j], Us[j * nb + n]));
-                const double2 u = Us[i * nb + n];
+                for (int j = 0; j < nb; ++j)
+                    t = cadd(t, cmul(__ldg(&rho[(long long)(i * nb + j) * Nk + k]), __ldg(&U[(long long)(j * nb + n) * Nk + k])));
+                const double2 u = __ldg(&U[(long long)(i * nb + n) * Nk + k]);
                 bl += u.x * t.x + u.y * t.y;  // Re(conj(u) t)
             }
-            atomicAdd(&acc[n], bl);
-        }
-        atomicAdd(&acc[nb + n], R[n * nb + n].x);
+        put(n, bl);
+        put(nb + n, on ? __ldg(&rho[(long long)(n * nb + n) * Nk + k]).x : 0.0);
     }
-    if (!v0) return;
     const double2* vs[3] = {v0, v1, v2};
-    double part[6] = {0, 0, 0, 0, 0, 0};
-    for (int p = threadIdx.x; p < P; p += blockDim.x) {
-        const int n = p / nb, l = p - (p / nb) * nb;
-        const double2 r = R[l * nb + n];
 #pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            const double2 c = cmul(vs[d][(long long)p * Nk + k], r);
-            part[2 * d] += c.x;
-            part[2 * d + 1] += c.y;
+    for (int d = 0; d < 3; ++d) {
+        double2 s = make_double2(0.0, 0.0);
+        if (v0 && on)
+            for (int n = 0; n < nb; ++n)
+                for (int l = 0; l < nb; ++l)
+                    s = cadd(s, cmul(__ldg(&vs[d][(long long)(n * nb + l) * Nk + k]), __ldg(&rho[(long long)(l * nb + n) * Nk + k])));
+        put(2 * nb + 2 * d, s.x);
+        put(2 * nb + 2 * d + 1, s.y);
+    }
+    __syncthreads();
+    for (int v = threadIdx.x; v < nacc; v += 128) mine[v] = red[0][v] + red[1][v] + red[2][v] + red[3][v];
+    __syncthreads();
+    observables_finish(mine, nacc, part, out, status, count);
+}
+
+// A CTA walks k points, rho_k and U_k in shared memory; its sums stay in
+// registers until the end.
+__global__ void __launch_bounds__(128) observables_kernel(
+    const double2* __restrict__ rho, const double2* __restrict__ U, const double2* __restrict__ v0,
+    const double2* __restrict__ v1, const double2* __restrict__ v2, int Nk, int nb, double* __restrict__ part,
+    double* __restrict__ out, const int* __restrict__ status, unsigned* __restrict__ count) {
+    extern __shared__ double2 so[];
+    const int P = nb * nb, nacc = 2 * nb + 6;
+    double2* R = so;
+    double2* Us = so + P;
+    double* mine = (double*)(so + 2 * P);              // [nacc]
+    double(*red)[6] = (double(*)[6])(mine + nacc);     // [4][6]
+    double bl = 0.0, wn = 0.0;  // of band n = threadIdx.x (nb <= 64 < 128 threads)
+    double vel[6] = {0, 0, 0, 0, 0, 0};
+    const double2* vs[3] = {v0, v1, v2};
+    for (int k = blockIdx.x; k < Nk; k += gridDim.x) {
+        for (int p = threadIdx.x; p < P; p += blockDim.x) {
+            R[p] = rho[(long long)p * Nk + k];
+            if (U) Us[p] = U[(long long)p * Nk + k];
         }
+        __syncthreads();
+        const int n = threadIdx.x;
+        if (n < nb) {
+            if (U)
+                for (int i = 0; i < nb; ++i) {
+                    double2 t = make_double2(0.0, 0.0);
+                    for (int j = 0; j < nb; ++j) t = cadd(t, cmul(R[i * nb + j], Us[j * nb + n]));
+                    const double2 u = Us[i * nb + n];
+                    bl += u.x * t.x + u.y * t.y;  // Re(conj(u) t)
+                }
+            wn += R[n * nb + n].x;
+        }
+        if (v0)
+            for (int p = threadIdx.x; p < P; p += blockDim.x) {
+                const int i = p / nb, l = p - (p / nb) * nb;
+                const double2 r = R[l * nb + i];
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    const double2 c = cmul(vs[d][(long long)p * Nk + k], r);
+                    vel[2 * d] += c.x;
+                    vel[2 * d + 1] += c.y;
+                }
+            }
+        __syncthreads();
     }
 #pragma unroll
     for (int q = 0; q < 6; ++q) {
-        double v = part[q];
-        for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
-        if ((threadIdx.x & 31) == 0) atomicAdd(&acc[2 * nb + q], v);
+        double v = vel[q];
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][q] = v;
     }
+    if (threadIdx.x < nb) {
+        mine[threadIdx.x] = bl;
+        mine[nb + threadIdx.x] = wn;
+    }
+    __syncthreads();
+    if (threadIdx.x < 6)
+        mine[2 * nb + threadIdx.x] = red[0][threadIdx.x] + red[1][threadIdx.x] + red[2][threadIdx.x] + red[3][threadIdx.x];
+    __syncthreads();
+    observables_finish(mine, nacc, part, out, status, count);
 }
 
 // plane position (digit-reversed order) of the natural R index (j0 N1 + j1) N2 + j2
@@ -1000,6 +1221,23 @@ int check_status(edus_handle* h) {
                     "a bounded wait in a kernel ran out (commutator_ws_kernel operand hand-over or "
                     "plane_rhs_persist_kernel bulk load): the results since the last synchronising call are invalid");
     }
+    return EDUS_OK;
+}
+
+// CTAs of the observables kernel
+int obs_grid(const edus_handle* h) { return h->nb <= 8 ? (h->Nk + 127) / 128 : std::min(h->Nk, 592); }
+
+// and its shared memory: rho_k, U_k, the sums and the warps' velocity sums
+int obs_smem(const edus_handle* h) { return (int)(2 * h->P * sizeof(double2) + (2 * h->nb + 6 + 24) * sizeof(double)); }
+
+int ensure_obsacc(edus_handle* h) {
+    if (h->obsacc) return EDUS_OK;
+    const size_t n = 2 * (size_t)h->nb + 6;
+    int rc;
+    if ((rc = dalloc(h, (void**)&h->obsacc, (n + 1 + n * obs_grid(h) + 1) * sizeof(double)))) return rc;
+    CU(h, cudaMemsetAsync(h->obsacc, 0, (n + 1 + n * obs_grid(h) + 1) * sizeof(double), h->stream));
+    if (cudaMallocHost((void**)&h->obs_host, (n + 1) * sizeof(double)) != cudaSuccess)
+        return fail(h, EDUS_ERR_NOMEM, "cudaMallocHost failed");
     return EDUS_OK;
 }
 
@@ -1229,7 +1467,7 @@ int edus_create(const edus_desc* desc, edus_handle** out) {
     if ((rc = set_smem(h, plane_rhs_kernel<true, kRadix89, 768>, h->smem_plane))) return bail(rc);
     if ((rc = set_smem(h, plane_rhs_kernel<false, kRadix89, 768>, h->smem_plane))) return bail(rc);
     if ((rc = set_smem(h, plane_to_R_kernel<kRadixAll, 256>, h->Nk * (int)sizeof(double2)))) return bail(rc);
-    if ((rc = set_smem(h, observables_kernel, 2 * h->P * (int)sizeof(double2)))) return bail(rc);
+    if ((rc = set_smem(h, observables_kernel, obs_smem(h)))) return bail(rc);
     if (h->Nk * (int)sizeof(double2) <= dev_smem &&
         (rc = set_smem(h, peierls_shift_kernel<kRadixAll, 256>, h->Nk * (int)sizeof(double2))))
         return bail(rc);
@@ -1337,6 +1575,7 @@ int edus_create(const edus_desc* desc, edus_handle** out) {
             h->use3 = true;
         }
     }
+    if (d.precision == EDUS_PREC_FP64 && (rc = resident_setup(h))) return bail(rc);
     std::vector<int> upair_host;
     if (herm_planes) {
         h->hplanes = true;
@@ -1468,6 +1707,7 @@ int edus_destroy(edus_handle* h) {
     for (cudaEvent_t e : h->prof_pool) cudaEventDestroy(e);
     for (void* p : h->allocs) cudaFree(p);
     for (int i = 0; i < 2; ++i) {
+        if (i == 0 && h->obs_host) cudaFreeHost(h->obs_host);
         if (h->field_host[i]) cudaFreeHost(h->field_host[i]);
         if (h->field_ev[i]) cudaEventDestroy(h->field_ev[i]);
     }
@@ -1730,8 +1970,7 @@ int edus_upload_observables(edus_handle* h, const double* U_k, const double* vel
     if (vel_k)
         for (int d = 0; d < 3; ++d)
             if ((rc = up(vel_k + 2 * h->S * d, &h->obsV[d]))) return rc;
-    if (!h->obsacc && (rc = dalloc(h, (void**)&h->obsacc, (2 * (size_t)h->nb + 6) * sizeof(double)))) return rc;
-    return EDUS_OK;
+    return ensure_obsacc(h);
 }
 
 int edus_observables(edus_handle* h, int b, int filled, double* pop_bloch, double* pop_wannier, double* vel) {
@@ -1740,8 +1979,8 @@ int edus_observables(edus_handle* h, int b, int filled, double* pop_bloch, doubl
     if (pop_bloch && !h->obsU) return fail(h, EDUS_ERR_ARG, "the Bloch populations need edus_upload_observables(U)");
     if (vel && !h->obsV[0]) return fail(h, EDUS_ERR_ARG, "the velocity needs edus_upload_observables(vel)");
     int rc;
-    if (!h->obsacc && (rc = dalloc(h, (void**)&h->obsacc, (2 * (size_t)h->nb + 6) * sizeof(double)))) return rc;
     CU(h, cudaSetDevice(h->d.device));
+    if ((rc = ensure_obsacc(h))) return rc;
     if (h->packed && (rc = unpack_state(h, b))) return rc;
     const int nacc = 2 * h->nb + 6;
     const double2* rho = h->y + (size_t)b * h->S;
@@ -1758,15 +1997,22 @@ int edus_observables(edus_handle* h, int b, int filled, double* pop_bloch, doubl
         CU(h, cudaGetLastError());
         rho = h->stage;
     }
-    CU(h, cudaMemsetAsync(h->obsacc, 0, nacc * sizeof(double), h->stream));
-    observables_kernel<<<h->Nk, 128, 2 * h->P * sizeof(double2), h->stream>>>(
-        rho, pop_bloch ? h->obsU : nullptr, vel ? h->obsV[0] : nullptr, h->obsV[1], h->obsV[2],
-        h->Nk, h->nb, h->obsacc);
+    double* part = h->obsacc + nacc + 1;
+    unsigned* count = (unsigned*)(part + (size_t)nacc * obs_grid(h));
+    if (h->nb <= 8)
+        observables_thread_kernel<<<obs_grid(h), 128, 0, h->stream>>>(rho, pop_bloch ? h->obsU : nullptr,
+                                                                      vel ? h->obsV[0] : nullptr, h->obsV[1], h->obsV[2],
+                                                                      h->Nk, h->nb, part, h->obsacc, h->flag, count);
+    else
+        observables_kernel<<<obs_grid(h), 128, obs_smem(h), h->stream>>>(
+            rho, pop_bloch ? h->obsU : nullptr, vel ? h->obsV[0] : nullptr, h->obsV[1], h->obsV[2], h->Nk, h->nb, part,
+            h->obsacc, h->flag, count);
     h->launches++;
     CU(h, cudaGetLastError());
-    std::vector<double> a(nacc);
-    CU(h, cudaMemcpyAsync(a.data(), h->obsacc, nacc * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+    // the sums and the status word in one copy
+    CU(h, cudaMemcpyAsync(h->obs_host, h->obsacc, (nacc + 1) * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     CU(h, cudaStreamSynchronize(h->stream));
+    const double* a = h->obs_host;
     const double inv = 1.0 / h->Nk;
     for (int n = 0; n < h->nb; ++n) {
         // Print_Population (Simulation.cpp:439-470): holes of the filled bands in the Bloch gauge
@@ -1775,7 +2021,7 @@ int edus_observables(edus_handle* h, int b, int filled, double* pop_bloch, doubl
     }
     if (vel)
         for (int q = 0; q < 6; ++q) vel[q] = a[2 * h->nb + q] * inv;
-    return check_status(h);
+    return a[nacc] != 0.0 ? check_status(h) : EDUS_OK;
 }
 
 int edus_efield(edus_handle* h, int b, double t, double* E) {
@@ -1964,6 +2210,7 @@ static int launch_plain_steps(edus_handle* h, int cnt) {
     const int B = h->B;
     const long long bs = (long long)h->S;
     int rc;
+    if (cnt > 0 && resident_active(h)) return launch_resident(h, cnt);
     for (int i = 0; i < cnt; ++i) {
         if (h->split && (!h->anchored || h->since_anchor >= h->anchor_every)) {
             if ((rc = anchor_split(h))) return rc;
@@ -2297,7 +2544,7 @@ int edus_step(edus_handle* h, int n) {
     const bool rk = h->d.solver == EDUS_SOLVER_RK;
     // small RK4 problems in the FP64 form: the same launches, 32 steps per
     // CUDA graph replay (captured once per call)
-    if (rk && !h->packed && !h->split && !h->profiling && n >= kGraphStepMin &&
+    if (rk && !h->packed && !h->split && !h->profiling && !resident_active(h) && n >= kGraphStepMin &&
         (size_t)h->S * h->B * sizeof(double2) <= kGraphStepBytes)
         return edus_sweep_step(&h, 1, n, 1);
     const int nst = rk ? 4 : 1;
@@ -2388,6 +2635,11 @@ int edus_sweep_step(edus_handle* const* hs, int n, int steps, int use_graph) {
     cudaGraphExec_t exec = nullptr;
     FusedSweep fs;
     int rc = EDUS_OK;
+    // the fused launches take the handles that do not step by the resident
+    // kernel; those that do run beside them, each on its own stream
+    std::vector<edus_handle*> hf, hown;
+    for (int i = 0; i < n; ++i) (fused && !resident_active(hs[i]) ? hf : hown).push_back(hs[i]);
+    std::vector<unsigned long long> chunk_launches(n, 0);
     auto cleanup = [&]() {
         if (s0) cudaStreamSynchronize(s0);
         fs.release();
@@ -2414,7 +2666,7 @@ int edus_sweep_step(edus_handle* const* hs, int n, int steps, int use_graph) {
             return fail(h0, EDUS_ERR_CUDA, std::string("sweep set-up: ") + cudaGetErrorString(pend));
         }
     }
-    if (fused && (rc = fused_setup(hs, n, C, fs))) {
+    if (!hf.empty() && (rc = fused_setup(hf.data(), (int)hf.size(), C, fs))) {
         cleanup();
         return rc;
     }
@@ -2425,17 +2677,21 @@ int edus_sweep_step(edus_handle* const* hs, int n, int steps, int use_graph) {
             const cudaError_t pend = cudaGetLastError();
             if (pend != cudaSuccess) return fail(h0, EDUS_ERR_CUDA, std::string("sweep, before launches: ") + cudaGetErrorString(pend));
         }
-        if (fused) return fused_launch_steps(hs, fs, cnt, s0);
         if (cudaEventRecord(fork, s0) != cudaSuccess) return fail(h0, EDUS_ERR_CUDA, "cudaEventRecord failed");
-        for (int i = 0; i < n; ++i) {
-            edus_handle* h = hs[i];
+        for (size_t i = 0; i < hown.size(); ++i) {
+            edus_handle* h = hown[i];
             if (cudaStreamWaitEvent(h->stream, fork, 0) != cudaSuccess)
                 return fail(h, EDUS_ERR_CUDA, "cudaStreamWaitEvent failed");
             int r;
             if ((r = launch_plain_steps(h, cnt))) return r;
-            if (cudaEventRecord(join[i], h->stream) != cudaSuccess || cudaStreamWaitEvent(s0, join[i], 0) != cudaSuccess)
+            if (cudaEventRecord(join[i], h->stream) != cudaSuccess)
                 return fail(h, EDUS_ERR_CUDA, "sweep join failed");
         }
+        int r;
+        if (!hf.empty() && (r = fused_launch_steps(hf.data(), fs, cnt, s0))) return r;
+        for (size_t i = 0; i < hown.size(); ++i)
+            if (cudaStreamWaitEvent(s0, join[i], 0) != cudaSuccess)
+                return fail(hown[i], EDUS_ERR_CUDA, "sweep join failed");
         return EDUS_OK;
     };
     for (int done = 0; done < steps && rc == EDUS_OK;) {
@@ -2475,6 +2731,7 @@ int edus_sweep_step(edus_handle* const* hs, int n, int steps, int use_graph) {
                 const cudaError_t ec = cudaStreamEndCapture(s0, &g);
                 for (int i = 0; i < n; ++i) {  // the capture ran nothing
                     hs[i]->t = t0[i];
+                    chunk_launches[i] = hs[i]->launches - l0[i];
                     hs[i]->launches = l0[i];
                 }
                 if (r || ec != cudaSuccess || cudaGraphInstantiate(&exec, g, 0) != cudaSuccess) {
@@ -2490,9 +2747,8 @@ int edus_sweep_step(edus_handle* const* hs, int n, int steps, int use_graph) {
             }
             for (int i = 0; i < n; ++i) {
                 for (int k = 0; k < C; ++k) hs[i]->t += hs[i]->d.dt;  // as the launches would
-                if (!fused) hs[i]->launches += 8LL * C;
+                hs[i]->launches += chunk_launches[i];
             }
-            if (fused) h0->launches += (unsigned long long)C * fused_launches_per_step(fs);
         } else {
             rc = launch_all(cnt);
         }

@@ -12,17 +12,10 @@
 #pragma once
 #include <cuda_runtime.h>
 #include "fft_plane.cuh"
+#include "stage_field.hpp"
 #include "tma.cuh"
 
 namespace edus {
-
-// Field of one solve at one stage: E (Cartesian, a.u.) and g = A^T E, so that
-// R.E = g . R_crys for the Gamma-centred crystal coordinates R_crys.
-struct StageField {
-    double E[3];
-    double g[3];
-    double ga[3];  // Peierls gauge: A.R = ga . R_crys with A(t) the vector potential
-};
 
 // Peierls phases of one stage, per solve b and axis: tab[b * ntab + rposoff_d + q]
 // = exp(i ga_d R_d(q)), R_d(q) the Gamma-centred coordinate of position q, so
