@@ -68,40 +68,78 @@ int nfail(int code, const std::string& msg) {
 
 size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
-// H1[p][k] = H0[k][p] + sum_d E_d xi_d[k][p] (the sequence the commutator
-// kernel uses), transposed into the plane layout.
-__global__ void prep_hamiltonian(const double2* __restrict__ H0, const double2* __restrict__ xi, double2* __restrict__ H1,
-                                 int Nk, int P, double e0, double e1, double e2) {
+// Every input into the plane layout, 32 x 32 tiles through shared memory (reads
+// and writes both coalesced), one launch; blockIdx.z picks the arrays:
+//   0  rho_pk[p][k] = rho[k][p]
+//   1  H1[p][k] = H0[k][p] + sum_d E_d xi_d[k][p] (the commutator's sequence)
+//   2  (HSEX) W (real part) and rho0 at the digit-reversed positions of the plane
+//      FFT, and rho0_nn(R=0) into r0diag
+// 14 bands on 48 x 48 with HSEX: 18.6 us; as three launches with strided reads
+// or writes 23.6 us and two more launch gaps.
+struct PrepArgs {
+    const double2 *rho, *H0, *xi, *W, *rho0;
+    double2 *rho_pk, *H1, *r0p, *r0diag;
+    double* Wp;
+    const int *fq0, *fq1, *fq2;
+    int N1, N2, Nk, nb;
+    double e[3];
+    int* status;
+};
+__global__ void __launch_bounds__(256) prep_inputs(PrepArgs a) {
+    __shared__ double2 tile[32][33];
+    __shared__ double wtile[32][33];
+    const int Nk = a.Nk, nb = a.nb, P = nb * nb, role = blockIdx.z;
     const long long S = (long long)Nk * P;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < S; i += (long long)gridDim.x * blockDim.x) {
-        const int k = (int)(i / P), p = (int)(i - (long long)(i / P) * P);
-        double2 h = H0[i];
-        if (e0 != 0.0) { const double2 x = xi[i]; h.x += e0 * x.x; h.y += e0 * x.y; }
-        if (e1 != 0.0) { const double2 x = xi[S + i]; h.x += e1 * x.x; h.y += e1 * x.y; }
-        if (e2 != 0.0) { const double2 x = xi[2 * S + i]; h.x += e2 * x.x; h.y += e2 * x.y; }
-        H1[(long long)p * Nk + k] = h;
+    const int k0 = blockIdx.x * 32, p0 = blockIdx.y * 32, lane = threadIdx.x, p = p0 + lane;
+    // a thread's four elements: every load is issued before any is used
+    double2 v[4], x[3][4];
+    bool on[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const int k = k0 + threadIdx.y + 8 * u;
+        on[u] = k < Nk && p < P;
+        if (!on[u]) continue;
+        const long long i = (long long)k * P + p;
+        if (role == 0) {
+            v[u] = __ldg(&a.rho[i]);
+        } else if (role == 1) {
+            v[u] = __ldg(&a.H0[i]);
+#pragma unroll
+            for (int d = 0; d < 3; ++d)
+                if (a.e[d] != 0.0) x[d][u] = __ldg(&a.xi[d * S + i]);
+        } else {
+            const int q2 = k % a.N2, t = k / a.N2, q1 = t % a.N1, q0 = t / a.N1;
+            const long long j = (((long long)a.fq0[q0] * a.N1 + a.fq1[q1]) * a.N2 + a.fq2[q2]) * P + p;
+            v[u] = __ldg(&a.rho0[j]);
+            x[0][u] = __ldg(&a.W[j]);
+        }
     }
-}
-
-// W (real part) and rho0 from [R][p] into the plane layout at the
-// digit-reversed positions of the plane FFT; rho0_nn(R=0) into r0diag.
-__global__ void prep_hsex(const double2* __restrict__ W, const double2* __restrict__ rho0, double* __restrict__ Wp,
-                          double2* __restrict__ r0p, double2* __restrict__ r0diag, const int* __restrict__ fq0,
-                          const int* __restrict__ fq1, const int* __restrict__ fq2, int N1, int N2, int Nk, int nb,
-                          int* __restrict__ status) {
-    const int P = nb * nb;
-    const long long S = (long long)Nk * P;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < S; i += (long long)gridDim.x * blockDim.x) {
-        const int p = (int)(i / Nk), pos = (int)(i - (long long)p * Nk);
-        const int q2 = pos % N2, t = pos / N2, q1 = t % N1, q0 = t / N1;
-        const long long iR = ((long long)fq0[q0] * N1 + fq1[q1]) * N2 + fq2[q2];
-        const double2 w = W[iR * P + p];
-        Wp[i] = w.x;
-        if (w.y != 0.0) *status = 1;  // refused: the output becomes NaN
-        r0p[i] = rho0[iR * P + p];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        if (!on[u]) continue;
+        if (role == 1) {
+#pragma unroll
+            for (int d = 0; d < 3; ++d)
+                if (a.e[d] != 0.0) {
+                    v[u].x += a.e[d] * x[d][u].x;
+                    v[u].y += a.e[d] * x[d][u].y;
+                }
+        } else if (role == 2) {
+            wtile[threadIdx.y + 8 * u][lane] = x[0][u].x;
+            if (x[0][u].y != 0.0) *a.status = 1;  // refused: the output becomes NaN
+        }
+        tile[threadIdx.y + 8 * u][lane] = v[u];
     }
-    if (blockIdx.x == 0)
-        for (int n = threadIdx.x; n < nb; n += blockDim.x) r0diag[n] = rho0[n * nb + n];
+    if (role == 2 && blockIdx.x == 0 && blockIdx.y == 0)
+        for (int n = threadIdx.y * 32 + lane; n < nb; n += 256) a.r0diag[n] = a.rho0[n * nb + n];
+    __syncthreads();
+    double2* dst = role == 0 ? a.rho_pk : (role == 1 ? a.H1 : a.r0p);
+    const int k = k0 + lane;
+    for (int r = threadIdx.y; r < 32; r += 8) {
+        if (k >= Nk || p0 + r >= P) continue;
+        dst[(long long)(p0 + r) * Nk + k] = tile[lane][r];
+        if (role == 2) a.Wp[(long long)(p0 + r) * Nk + k] = wtile[lane][r];
+    }
 }
 
 // The evaluation's two stage fields (by value: no host copy), a cleared
@@ -207,7 +245,8 @@ extern "C" int edus_rhs_noalloc(const int grid[3], int nbands, int coulomb, cons
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return nfail(EDUS_ERR_CUDA, std::string("cudaGetDevice: ") + cudaGetErrorString(e));
     if (dev < 0 || dev >= kMaxDevices) return nfail(EDUS_ERR_UNSUPPORTED, "edus_rhs_noalloc: device ordinal too large");
-    int dev_smem = 0;
+    int dev_smem = 0, sm_count = 0;
+    cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
     cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     if (plane_smem > (size_t)dev_smem || comm_smem > (size_t)dev_smem)
         return nfail(EDUS_ERR_UNSUPPORTED, "edus_rhs_noalloc: k grid or band count too large for shared memory");
@@ -225,6 +264,8 @@ extern "C" int edus_rhs_noalloc(const int grid[3], int nbands, int coulomb, cons
             const int lim = dev_smem;
             if ((e = cudaFuncSetAttribute(plane_rhs_kernel<true, kRadixAll, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim)) != cudaSuccess ||
                 (e = cudaFuncSetAttribute(plane_rhs_kernel<false, kRadixAll, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim)) != cudaSuccess ||
+                (e = cudaFuncSetAttribute(plane_rhs_kernel<true, kRadixCommon, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim)) != cudaSuccess ||
+                (e = cudaFuncSetAttribute(plane_rhs_kernel<false, kRadixCommon, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim)) != cudaSuccess ||
                 (e = cudaFuncSetAttribute(commutator_kernel<MODE_RHS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim)) != cudaSuccess ||
                 (e = cudaFuncSetAttribute(commutator_kernel<MODE_RHS, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim)) != cudaSuccess ||
                 (e = cudaFuncSetAttribute(commutator_mma_kernel<MODE_RHS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim)) != cudaSuccess ||
@@ -282,26 +323,46 @@ extern "C" int edus_rhs_noalloc(const int grid[3], int nbands, int coulomb, cons
     set_call_state<<<1, 64, 0, stream>>>(d_field, hf[0], hf[1], diag0, nb, d_status);
     NA_CU(cudaGetLastError());
 
-    const int nthr = 256;
-    const int nblk = (int)std::min<size_t>((S + nthr - 1) / nthr, 148 * 16);
-    dim3 tb(32, 8), tg((Nk + 31) / 32, (P + 31) / 32);
-    transpose_kp_to_pk<<<tg, tb, 0, stream>>>((const double2*)in_k, rho_pk, Nk, P);
-    prep_hamiltonian<<<nblk, nthr, 0, stream>>>((const double2*)H0_k, (const double2*)xi_k, H1, Nk, P, efield[0],
-                                                 efield[1], efield[2]);
-    if (coulomb)
-        prep_hsex<<<nblk, nthr, 0, stream>>>((const double2*)W_R, (const double2*)rho0_R, Wp, r0p, r0diag,
-                                             d_fq + fqoff[0], d_fq + fqoff[1], d_fq + fqoff[2], N[1], N[2], Nk, nb,
-                                             d_status);
+    dim3 tb(32, 8);
+    PrepArgs pa{};
+    pa.rho = (const double2*)in_k;
+    pa.H0 = (const double2*)H0_k;
+    pa.xi = (const double2*)xi_k;
+    pa.W = (const double2*)W_R;
+    pa.rho0 = (const double2*)rho0_R;
+    pa.rho_pk = rho_pk;
+    pa.H1 = H1;
+    pa.r0p = r0p;
+    pa.r0diag = r0diag;
+    pa.Wp = Wp;
+    pa.fq0 = d_fq + fqoff[0];
+    pa.fq1 = d_fq + fqoff[1];
+    pa.fq2 = d_fq + fqoff[2];
+    pa.N1 = N[1];
+    pa.N2 = N[2];
+    pa.Nk = Nk;
+    pa.nb = nb;
+    for (int d = 0; d < 3; ++d) pa.e[d] = efield[d];
+    pa.status = d_status;
+    prep_inputs<<<dim3((Nk + 31) / 32, (P + 31) / 32, coulomb ? 3 : 2), tb, 0, stream>>>(pa);
     NA_CU(cudaGetLastError());
     dim3 pg(P, 1);
-    if (coulomb)
-        plane_rhs_kernel<true, kRadixAll, 512><<<pg, 512, plane_smem, stream>>>(rho_pk, 0, G, Hee, 0, r0p, Wp, diag0,
-                                                                                 d_field, d_roots, d_rpos, plan, nb,
-                                                                                 1.0 / Nk, nullptr, nullptr, 0);
-    else
-        plane_rhs_kernel<false, kRadixAll, 512><<<pg, 512, plane_smem, stream>>>(rho_pk, 0, G, Hee, 0, r0p, Wp, diag0,
-                                                                                  d_field, d_roots, d_rpos, plan, nb,
-                                                                                  1.0 / Nk, nullptr, nullptr, 0);
+    // More planes than SMs: 256 threads, so that two CTAs (128 registers a
+    // thread) share an SM and the planes run in one wave where they would take
+    // two (196 planes of 48 x 48 with HSEX: 50 -> 32 us); else 512 threads a plane.
+    const bool wide = plane_launch(plan).variant == 2;  // radix 11 or 13
+    const int threads = P > sm_count ? 256 : 512;
+    auto run_planes = [&](auto kernel) {
+        kernel<<<pg, threads, plane_smem, stream>>>(rho_pk, 0, G, Hee, 0, r0p, Wp, diag0, d_field, d_roots, d_rpos, plan,
+                                                    nb, 1.0 / Nk, nullptr, nullptr, 0, nullptr, 0);
+    };
+    if (coulomb) {
+        if (wide) run_planes(plane_rhs_kernel<true, kRadixAll, 512>);
+        else run_planes(plane_rhs_kernel<true, kRadixCommon, 512>);
+    } else {
+        if (wide) run_planes(plane_rhs_kernel<false, kRadixAll, 512>);
+        else run_planes(plane_rhs_kernel<false, kRadixCommon, 512>);
+    }
     NA_CU(cudaGetLastError());
     StageArgs a{};
     a.rho = rho_pk;
