@@ -201,6 +201,13 @@ __global__ void __launch_bounds__(32 * (2 + 2 * (TILES == 3 ? 8 : 4)), 1)
                 tma_load_4d(dst, &maps.m[2], x, b, full_e);
                 if (NEED_Y) tma_load_4d(dst + g.uarr_bytes, &maps.m[3], x, b, full_e);
                 if (NEED_A) tma_load_4d(dst + 2 * g.uarr_bytes, &maps.m[4], x, b, full_e);
+                if (MODE == MODE_AB) {
+                    // the update warps read the history directly: the next tile's to L2
+                    const int un = u + gridDim.x;
+                    if (j + 1 < nit)
+                        for (int q = 1; q < a.order; ++q)
+                            tma_prefetch_4d(&maps.m[4 + q], 2 * (un - un / ntu * ntu) * TKU, un / ntu);
+                }
             }
             issued = j + 1;
         }
@@ -313,6 +320,19 @@ __global__ void __launch_bounds__(32 * (2 + 2 * (TILES == 3 ? 8 : 4)), 1)
         const double2* Ys = (const double2*)(es + g.uarr_bytes);
         const double2* As = (const double2*)(es + 2 * g.uarr_bytes);
         for (int h = 0; h < 2; ++h) {
+            // Adams-Bashforth: the history of the next element is always in
+            // flight, the first one's while this half's products finish
+            double2 hn[4];
+            auto request = [&](int idx) {
+                const int kq = 2 * h + (idx & 1);
+                if (MODE == MODE_AB && idx < P * TK && k0 + kq < Nk) {
+                    const long long e = boff + (long long)(idx >> 1) * Nk + k0 + kq;
+#pragma unroll
+                    for (int q = 1; q < 5; ++q)
+                        if (q < a.order) hn[q - 1] = __ldg(&a.hist[q][e]);
+                }
+            };
+            request(ew * 32 + lane);
             if (!warp_wait(&full_c[h], par, kWaitPolls) || (h == 0 && !warp_wait(full_e, par, kWaitPolls))) {
                 if (lane == 0) atomicOr(status, 1);
                 return;
@@ -320,6 +340,12 @@ __global__ void __launch_bounds__(32 * (2 + 2 * (TILES == 3 ? 8 : 4)), 1)
             const double2* Cs = (const double2*)(base + g.off_c + h * g.arr_bytes);  // [TK][nb][CW]
             for (int idx = ew * 32 + lane; idx < P * TK; idx += NE * 32) {
                 const int p = idx >> 1, kk = idx & 1, kq = 2 * h + kk;
+                double2 hc[4];
+                if (MODE == MODE_AB) {
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) hc[q] = hn[q];
+                    request(idx + NE * 32);
+                }
                 if (k0 + kq >= Nk) continue;
                 const long long e = boff + (long long)p * Nk + k0 + kq;
                 const int eu = p * TKU + kq;  // in the update operands [P][TKU]
@@ -343,10 +369,9 @@ __global__ void __launch_bounds__(32 * (2 + 2 * (TILES == 3 ? 8 : 4)), 1)
                 } else if (MODE == MODE_AB) {
                     a.hist[0][e] = f;
                     double2 yy = make_double2(yv.x + a.c[0] * f.x, yv.y + a.c[0] * f.y);
-                    for (int qh = 1; qh < a.order; ++qh) {
-                        const double2 fq = a.hist[qh][e];
-                        yy = make_double2(yy.x + a.c[qh] * fq.x, yy.y + a.c[qh] * fq.y);
-                    }
+#pragma unroll
+                    for (int qh = 1; qh < 5; ++qh)
+                        if (qh < a.order) yy = make_double2(yy.x + a.c[qh] * hc[qh - 1].x, yy.y + a.c[qh] * hc[qh - 1].y);
                     a.y[e] = yy;
                 }
             }

@@ -588,9 +588,10 @@ int launch_ws(edus_handle* h, const StageArgs& a, int nbatch) {
     const int ntiles = ((h->Nk + g.TKU - 1) / g.TKU) * nbatch;  // update tiles
     const int grid = std::min(ntiles, h->ws_grid);
     OperandMaps maps;
-    const void* src[5] = {a.Hee, a.rho, a.G, a.y ? (const void*)a.y : (const void*)a.G,
+    const void* src[9] = {a.Hee, a.rho, a.G, a.y ? (const void*)a.y : (const void*)a.G,
                           a.acc ? (const void*)a.acc : (const void*)a.G};
-    for (int i = 0; i < 5; ++i) {
+    for (int q = 1; q < 5; ++q) src[4 + q] = MODE == MODE_AB && q < a.order ? (const void*)a.hist[q] : (const void*)a.G;
+    for (int i = 0; i < 9; ++i) {
         const CUtensorMap* m = operand_map(h, src[i], nbatch, i < 2);
         if (!m) return fail(h, EDUS_ERR_CUDA, "cuTensorMapEncodeTiled failed for a commutator operand");
         maps.m[i] = *m;

@@ -9,10 +9,11 @@
 
 namespace edus {
 
-// Operand tensor maps of one launch (H, rho, G, y, acc), each describing a
-// [B][P][Nk] complex array as the 4-D tensor {2 Nk, nb, nb, B} of doubles.
+// Operand tensor maps of one launch (H, rho, G, y, acc, and the Adams-Bashforth
+// history hist[1] ..), each describing a [B][P][Nk] complex array as the 4-D
+// tensor {2 Nk, nb, nb, B} of doubles.
 struct OperandMaps {
-    CUtensorMap m[5];
+    CUtensorMap m[9];
 };
 
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
@@ -53,6 +54,14 @@ __device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, i
         "[%6];\n" ::"r"(smem_u32(dst)),
         "l"(reinterpret_cast<unsigned long long>(map)), "r"(x), "r"(0), "r"(0), "r"(b), "r"(smem_u32(bar))
         : "memory");
+}
+
+// the same box into L2 only
+__device__ __forceinline__ void tma_prefetch_4d(const CUtensorMap* map, int x, int b) {
+    asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];\n" ::"l"(
+                     reinterpret_cast<unsigned long long>(map)),
+                 "r"(x), "r"(0), "r"(0), "r"(b)
+                 : "memory");
 }
 
 // Untiled bulk copy global -> shared (no multicast): addresses 16-byte aligned,
