@@ -1,7 +1,7 @@
 // Warp-specialised, TMA-fed persistent commutator for the fused-Hamiltonian
-// HSEX path (12 <= nb <= 24): the contract of commutator_mma_kernel with
+// paths (12 <= nb <= 24): the contract of commutator_mma_kernel with
 // FH = true (Hee holds H0 + E.xi + Hee; the Hartree diagonal hh is added
-// here), with the tensor-core products overlapping the stage update and the
+// here, none without HSEX: hartree == nullptr), with the tensor-core products overlapping the stage update and the
 // copies.
 //
 // A CTA walks update tiles of 4 consecutive k points (u = blockIdx.x,
@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(32 * (2 + 2 * (TILES == 3 ? 8 : 4)), 1)
             double2* hh = (double2*)(dst + g.hh_off);
             if (b != last_b) {
                 hreg = make_double2(0.0, 0.0);
-                if (lane < nb)
+                if (a.hartree && lane < nb)
                     for (int m = 0; m < nb; ++m)
                         hreg = cadd(hreg, cmul(__ldg(&a.hartree[lane * nb + m]),
                                                csub(__ldg(&a.diag0[b * nb + m]), __ldg(&a.rho0diag[m]))));

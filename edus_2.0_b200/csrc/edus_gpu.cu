@@ -85,6 +85,10 @@ struct edus_handle {
     // box kind): kind 0 the dense box, kind 1 the zero-padded box of the
     // product operands
     bool comm_ws = false;
+    // the same kernel without HSEX, for states too large for L2: H0 + E.xi is
+    // written to Hee when E changes (hamiltonian_kernel)
+    bool ws_ipa = false;
+    const StageField* prev_field = nullptr;  // field of the stage launched before, when Hee holds its H
     int ws_grid = 0;
     // Peierls gauge (edus_set_peierls): per-axis phase tables of the stage
     // ([B][ntab]) and each solve's vector-potential integrator (A, last time)
@@ -582,6 +586,46 @@ const CUtensorMap* operand_map(edus_handle* h, const void* base, int nbatch, boo
     return &(h->tmaps[key] = m);
 }
 
+// H[b][p][k] = H0 + sum_d E_d xi_d of every solve's field, unless the stage
+// before had the same field (stages 2 and 3 of RK4 share their time, as do
+// stage 4 and the next step's first): then H is there already.
+__global__ void __launch_bounds__(256) hamiltonian_kernel(StageArgs a, const StageField* __restrict__ prev,
+                                                          double2* __restrict__ H) {
+    const int b = blockIdx.y;
+    const StageField F = a.field[b];
+    if (prev) {
+        const StageField G = prev[b];
+        if (F.E[0] == G.E[0] && F.E[1] == G.E[1] && F.E[2] == G.E[2]) return;
+    }
+    const bool e0 = F.E[0] != 0.0, e1 = F.E[1] != 0.0, e2 = F.E[2] != 0.0;
+    const long long mb = (long long)b * a.mstride, ob = (long long)b * a.bstride;
+    constexpr int U = 4;
+    const long long T = (long long)gridDim.x * blockDim.x;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < a.bstride; i += U * T) {
+        double2 h[U], x0[U], x1[U], x2[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const long long j = i + u * T;
+            if (j < a.bstride) {
+                h[u] = __ldg(&a.H0[mb + j]);
+                if (e0) x0[u] = __ldg(&a.xi[0][mb + j]);
+                if (e1) x1[u] = __ldg(&a.xi[1][mb + j]);
+                if (e2) x2[u] = __ldg(&a.xi[2][mb + j]);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const long long j = i + u * T;
+            if (j >= a.bstride) continue;
+            double2 v = h[u];
+            if (e0) { v.x += F.E[0] * x0[u].x; v.y += F.E[0] * x0[u].y; }
+            if (e1) { v.x += F.E[1] * x1[u].x; v.y += F.E[1] * x1[u].y; }
+            if (e2) { v.x += F.E[2] * x2[u].x; v.y += F.E[2] * x2[u].y; }
+            H[ob + j] = v;
+        }
+    }
+}
+
 template <int MODE>
 int launch_ws(edus_handle* h, const StageArgs& a, int nbatch) {
     const WsGeom g = ws_geometry(h->nb);
@@ -616,6 +660,16 @@ int launch_comm_mode(edus_handle* h, const StageArgs& a, int nbatch, bool fuse) 
     if (fh && h->comm_ws) {
         int rc;
         if ((rc = launch_ws<MODE>(h, a, nbatch))) return rc;
+    } else if (!fh && fuse && h->ws_ipa) {
+        // 16 CTAs of 4 elements a thread cover 16 k elements; more than the SMs hold queue up
+        const unsigned gx = (unsigned)std::min<long long>((a.bstride + 1023) / 1024, 148LL * 16);
+        hamiltonian_kernel<<<dim3(gx, nbatch), 256, 0, h->stream>>>(a, h->prev_field, h->Hee);
+        h->launches++;
+        int rc;
+        StageArgs aw = a;
+        aw.Hee = h->Hee;
+        aw.hartree = nullptr;
+        if ((rc = launch_ws<MODE>(h, aw, nbatch))) return rc;
     } else if (fh && !h->d.coulomb) {
         if (h->comm_mma)
             commutator_mma_kernel<MODE, false, true><<<grid, h->comm_threads, h->smem_comm, h->stream>>>(a);
@@ -1486,7 +1540,10 @@ int edus_create(const edus_desc* desc, edus_handle** out) {
     if ((rc = set_smem(h, commutator_mma_kernel<M, false, true>, smem_cmax))) return bail(rc);
     SETC(MODE_RHS) SETC(MODE_RK1) SETC(MODE_RK2) SETC(MODE_RK3) SETC(MODE_RK4) SETC(MODE_AB)
 #undef SETC
-    if (d.coulomb && ws_supported(h->nb) && tensor_map_encoder()) {
+    // Without HSEX from 32 MB of state (all solves) up: below, the states and
+    // models stay in L2 and the tensor-core kernel's direct loads do as well.
+    const bool want_ws_ipa = !d.coulomb && d.precision == EDUS_PREC_FP64 && h->S * h->B * sizeof(double2) >= (32u << 20);
+    if ((d.coulomb || want_ws_ipa) && ws_supported(h->nb) && tensor_map_encoder()) {
         const WsGeom wg = ws_geometry(h->nb);
         if ((int)wg.smem <= dev_smem) {
 #define SETW(M)                                                                                           \
@@ -1508,7 +1565,7 @@ int edus_create(const edus_desc* desc, edus_handle** out) {
             int nsm = 0;
             cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, d.device);
             if (per_sm > 0 && nsm > 0) {
-                h->comm_ws = true;
+                (d.coulomb ? h->comm_ws : h->ws_ipa) = true;
                 h->ws_grid = per_sm * nsm;
             }
         }
@@ -1549,6 +1606,7 @@ int edus_create(const edus_desc* desc, edus_handle** out) {
         TRY_ALLOC(h->rho0diag, h->nb * sizeof(double2));
         TRY_ALLOC(h->diag0, (size_t)h->B * h->nb * sizeof(double2));
     }
+    if (h->ws_ipa) TRY_ALLOC(h->Hee, SBb);
     TRY_ALLOC(h->roots, roots.size() * sizeof(double2));
     TRY_ALLOC(h->rpos, rpos.size() * sizeof(double));
     TRY_ALLOC(h->field, (size_t)h->chunk * 4 * h->B * sizeof(StageField));
@@ -2232,7 +2290,10 @@ static int launch_plain_steps(edus_handle* h, int cnt) {
                 a.field = fs + (size_t)s * B;
                 a.c[0] = c0[s];
                 a.c[1] = c1[s];
-                if ((rc = launch_comm(h, MODE_RK1 + s, a, B))) return rc;
+                h->prev_field = i + s > 0 ? a.field - B : nullptr;
+                rc = launch_comm(h, MODE_RK1 + s, a, B);
+                h->prev_field = nullptr;
+                if (rc) return rc;
             }
         } else {
             if ((rc = launch_plane(h, h->y, bs, h->G, h->Hee, bs, fs, B))) return rc;
@@ -2824,6 +2885,8 @@ int edus_autotune(edus_handle* h, int* plane_threads, int* comm_tensor) {
             a.rho = h->y;
             a.field = df;
             a.out = h->stage;
+            const bool keep_ws = h->ws_ipa;
+            h->ws_ipa = false;  // the two kernels compared here also step the fused sweep
             float best = 1e30f;
             bool best_mma = h->comm_mma;
             for (int mma = 0; mma < 2; ++mma) {
@@ -2847,6 +2910,7 @@ int edus_autotune(edus_handle* h, int* plane_threads, int* comm_tensor) {
             h->TK = best_mma ? mg.TK : cg.TK;
             h->comm_threads = best_mma ? 256 : cg.threads;
             h->smem_comm = (int)(best_mma ? mg.smem : cg.smem);
+            h->ws_ipa = keep_ws;
         }
         if (comm_tensor) *comm_tensor = h->comm_mma ? 1 : 0;
     }
