@@ -661,7 +661,6 @@ int launch_comm_mode(edus_handle* h, const StageArgs& a, int nbatch, bool fuse) 
         int rc;
         if ((rc = launch_ws<MODE>(h, a, nbatch))) return rc;
     } else if (!fh && fuse && h->ws_ipa) {
-        // 16 CTAs of 4 elements a thread cover 16 k elements; more than the SMs hold queue up
         const unsigned gx = (unsigned)std::min<long long>((a.bstride + 1023) / 1024, 148LL * 16);
         hamiltonian_kernel<<<dim3(gx, nbatch), 256, 0, h->stream>>>(a, h->prev_field, h->Hee);
         h->launches++;
@@ -1540,9 +1539,9 @@ int edus_create(const edus_desc* desc, edus_handle** out) {
     if ((rc = set_smem(h, commutator_mma_kernel<M, false, true>, smem_cmax))) return bail(rc);
     SETC(MODE_RHS) SETC(MODE_RK1) SETC(MODE_RK2) SETC(MODE_RK3) SETC(MODE_RK4) SETC(MODE_AB)
 #undef SETC
-    // Without HSEX from 32 MB of state (all solves) up: below, the states and
-    // models stay in L2 and the tensor-core kernel's direct loads do as well.
-    const bool want_ws_ipa = !d.coulomb && d.precision == EDUS_PREC_FP64 && h->S * h->B * sizeof(double2) >= (32u << 20);
+    // Without HSEX from 12 MB of state (all solves) up: below, the extra launch
+    // that writes H0 + E.xi costs as much as the tiles it relieves.
+    const bool want_ws_ipa = !d.coulomb && d.precision == EDUS_PREC_FP64 && h->S * h->B * sizeof(double2) >= (12u << 20);
     if ((d.coulomb || want_ws_ipa) && ws_supported(h->nb) && tensor_map_encoder()) {
         const WsGeom wg = ws_geometry(h->nb);
         if ((int)wg.smem <= dev_smem) {

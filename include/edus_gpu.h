@@ -181,11 +181,15 @@ int edus_get_time(const edus_handle* h, double* t);
 int edus_rhs(edus_handle* h, double t, const double* in_k, double* out_k);
 
 /* Advance every solve by n steps (DESolver::Propagate(n), DESolver.hpp:238-242).
- * Asynchronous: returns once the work is queued.  Exception: an RK4 handle in
- * the FP64 form whose state (all solves) is at most 16 MB, profiling off, with
- * n >= 512, steps as edus_sweep_step of that one handle with use_graph 1 (the
- * same launches, 32 steps per CUDA graph replay, for small problems whose
- * steps are dominated by launch overhead) and returns once they are done. */
+ * Asynchronous: returns once the work is queued.  Small problems (FP64 form,
+ * length gauge, R-space gradient, profiling off) step in one launch per 256
+ * steps, a cluster of CTAs per solve holding it in shared memory; the choice
+ * follows an estimate of both forms' time from the grid, the band count and the
+ * batch.  Exception to the asynchrony: an RK4 handle in the FP64 form that does
+ * not step that way, whose state (all solves) is at most 16 MB, profiling off,
+ * with n >= 512, steps as edus_sweep_step of that one handle with use_graph 1
+ * (the same launches, 32 steps per CUDA graph replay) and returns once they are
+ * done. */
 int edus_step(edus_handle* h, int n);
 
 /* Advance n handles (one device, FP64 form) by `steps` steps together.
@@ -202,8 +206,11 @@ int edus_step(edus_handle* h, int n);
  *                  plane or k tile) are taken largest first from a counter;
  *                  chunks captured into a CUDA graph.  RK4, independent
  *                  particles, R-space gradient, length gauge (else
- *                  EDUS_ERR_UNSUPPORTED).  A solve's result equals stepping
- *                  its handle alone.
+ *                  EDUS_ERR_UNSUPPORTED).  Handles that step in one launch of
+ *                  their own (edus_step) run beside the fused launches.
+ * A solve's result equals stepping its handle alone (in the fused form to
+ * rounding, where the handle alone takes other kernels: many CTAs a plane, or
+ * the TMA-fed commutator of large states).
  * Synchronous.  No reference counterpart. */
 int edus_sweep_step(edus_handle* const* hs, int n, int steps, int use_graph);
 
