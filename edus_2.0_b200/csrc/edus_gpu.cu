@@ -859,7 +859,12 @@ int resident_setup(edus_handle* h) {
             h->res = g;
         }
     }
-    if (best > 1e29) return EDUS_OK;
+    // The launches per stage instead: two kernels (four where planes are spread
+    // over many CTAs) of 4.5-5 us each when nothing but latency counts, and ten
+    // array passes over the solves' states at about 2 TB/s.
+    const double launches_us = (h->use3 ? 20.0 : 9.0) + 160.0 * (double)h->S * h->B / 2.0e6;
+    const double own_us = 1.2 * best / 1900.0;  // a margin of 20% to the estimate
+    if (own_us >= launches_us) return EDUS_OK;
     int rc;
     if ((rc = set_smem(h, k, (int)h->res.smem))) return rc;
     if (h->res.CS > 8) CU(h, cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
@@ -870,12 +875,8 @@ int resident_setup(edus_handle* h) {
         cudaGetLastError();  // the device cannot place such a cluster: the launches per stage remain
         return EDUS_OK;
     }
-    // The launches per stage instead: two kernels (four where planes are spread
-    // over many CTAs) of 4.5-5 us each when nothing but latency counts, and ten
-    // array passes over the solves' states at about 2 TB/s.
     const double waves = std::ceil((double)h->B / clusters);
-    const double launches_us = (h->use3 ? 20.0 : 9.0) + 160.0 * (double)h->S * h->B / 2.0e6;
-    h->res_ok = 1.2 * best * waves / 1900.0 < launches_us;
+    h->res_ok = own_us * waves < launches_us;
     return EDUS_OK;
 }
 

@@ -4,7 +4,7 @@
 // kernel launches.
 //
 // What bounds such a problem is latency: a stage of the two-band chain (64 k
-// points) moves 4 KB and took 8.5 us as two launches, 4.2 us here; of two bands
+// points) moves 4 KB and took 8.5 us as two launches, 4.6 us here; of two bands
 // on 50 x 50 about 22 us as four launches, 11 us here; with HSEX on 40 x 40 26 us
 // and 12 us.
 //

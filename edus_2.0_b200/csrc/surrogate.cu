@@ -387,8 +387,8 @@ __device__ __forceinline__ void team_sync() {
 // 128 batch rows through the network and, with TRAIN, back, by a cluster of four
 // CTAs.  CTA j computes columns 32 j .. 32 j + 31 of every 128-wide layer block: its
 // share of the products (N = 32), of GELU and its derivative (erff and expf, the
-// largest part of the time: one CTA a row block, 4096 rows on 32 SMs, took 59 us;
-// four, 26 us) and of the loads and stores.  It writes its columns of an
+// largest part of the time: one CTA a row block, 4096 rows on 32 SMs, took 84 us;
+// four, 42 us) and of the loads and stores.  It writes its columns of an
 // activation or gradient block into all four CTAs' shared memory, so each holds
 // the whole block as the operand of its next product; one cluster barrier a
 // product orders this.  Buffers rotate: when a CTA writes block i it has passed
@@ -833,7 +833,7 @@ __global__ void mlp_pack_kernel(MlpShape s, const float* __restrict__ w, __nv_bf
 // eight inputs of one output of a weight tile, so its BF16 weights are one 16-byte
 // row of a core matrix and neighbouring threads read neighbouring outputs (one
 // parameter a thread, with 2-byte stores into the blocks, took 18 us for 99 k
-// parameters; this way 12).  The next blocks: a thread per bias; the last sums the loss.
+// parameters; this way 8).  The next blocks: a thread per bias; the last sums the loss.
 struct AdamArgs {
     float lr, b1, b2, eps, c1, c2;
 };
