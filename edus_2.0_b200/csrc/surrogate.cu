@@ -71,12 +71,22 @@ __device__ __forceinline__ bool mbar_wait_parity(unsigned long long* bar, unsign
     return false;
 }
 
+constexpr int kMlpPolls = 1 << 22;
+// False if the wait ran out after `polls`; what was waited for is then awaited
+// once more (bounded), so that no copy or product of this CTA is in flight when
+// the caller reports the failure and goes on.
+__device__ __forceinline__ bool mbar_wait_drain(unsigned long long* bar, unsigned parity, int polls) {
+    if (mbar_wait_parity(bar, parity, polls)) return true;
+    mbar_wait_parity(bar, parity, kMlpPolls);
+    return false;
+}
+
 __global__ void __launch_bounds__(128) gemm_bf16_kernel(int M, int N, int K, const __nv_bfloat16* __restrict__ A,
                                                        long long a_rs, long long a_cs,
                                                        const __nv_bfloat16* __restrict__ B, long long b_rs,
                                                        long long b_cs, float* __restrict__ C, int ldc,
                                                        const float* __restrict__ bias, int accumulate,
-                                                       int* __restrict__ status) {
+                                                       int* __restrict__ status, int polls) {
     __shared__ __align__(1024) __nv_bfloat16 As[UM * UK];  // 16 KB
     __shared__ __align__(1024) __nv_bfloat16 Bs[UN * UK];  // 16 KB
     __shared__ __align__(8) unsigned long long mbar;
@@ -132,11 +142,7 @@ __global__ void __launch_bounds__(128) gemm_bf16_kernel(int M, int N, int K, con
                          : "memory");
         }
         // the MMAs have read the operands (and written TMEM) once the phase completes
-        if (!mbar_wait_parity(&mbar, phase, 1 << 24)) {
-            // give up: report, wait (bounded again) for the MMAs in flight, skip the rest
-            ok = false;
-            mbar_wait_parity(&mbar, phase, 1 << 24);
-        }
+        if (!mbar_wait_drain(&mbar, phase, polls)) ok = false;  // give up: report, skip the rest
         phase ^= 1u;
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
         if (__syncthreads_or(!ok)) {
@@ -232,10 +238,21 @@ __global__ void colsum_kernel(const float* __restrict__ dz, float* __restrict__ 
     for (int i = 0; i < rows; ++i) s += dz[(long long)i * cols + j];
     db[j] = s;
 }
+// An update leaves weights and moments alone when a wait ran out in the kernels
+// that made its gradients (or in an earlier step's, not reported yet): status
+// stays set until the host reads it, and `skipped` counts the training steps
+// that were left out, which the host takes back from its step count.
+__device__ __forceinline__ bool update_skipped(const int* status, int* skipped, bool training) {
+    if (!*status) return false;
+    if (training && blockIdx.x == 0 && threadIdx.x == 0) ++*skipped;
+    return true;
+}
+
 // Adam on the FP32 master weights, refreshing their BF16 copy
 __global__ void adam_kernel(float* __restrict__ w, __nv_bfloat16* __restrict__ wb, const float* __restrict__ g,
                             float* __restrict__ m, float* __restrict__ v, long long n, float lr, float b1, float b2,
-                            float eps, float c1, float c2) {
+                            float eps, float c1, float c2, const int* __restrict__ status, int* __restrict__ skipped) {
+    if (update_skipped(status, skipped, true)) return;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         const float gi = g[i];
         const float mi = b1 * m[i] + (1.f - b1) * gi;
@@ -284,7 +301,6 @@ constexpr int kDwStages = 5;
 constexpr unsigned kDwStage = kBlkBytes + kGrp * 2u;  // a dz block and an activation column group
 constexpr size_t kDwSmem = (size_t)kDwStages * kDwStage + 1024;
 constexpr unsigned kBiasStage = 128 * 32 * 4;  // 128 rows x 32 outputs of dz in FP32
-constexpr int kMlpPolls = 1 << 22;
 
 __device__ __forceinline__ int blk_off(int r, int c) { return (r >> 3) * 1024 + (c >> 3) * 64 + (r & 7) * 8 + (c & 7); }
 __device__ __forceinline__ int act_off(int r, int c) {
@@ -365,6 +381,7 @@ struct MlpRowsArgs {
     float* lossp;              // [row block][4] (TRAIN)
     float scale;               // 1 / (B n_out)
     int* status;
+    int polls;                 // limit of every wait
 };
 
 constexpr int kTeam = 4;  // CTAs of a row block, a column group each
@@ -400,8 +417,8 @@ __device__ __forceinline__ void team_sync() {
 // Tensor-memory columns: the pre-activations of the hidden layers at 0, 32, 64,
 // the output block at 96; backward, the gradient of a layer's activations takes
 // the columns of the layer above it.  Every wait is bounded; one that runs out
-// sets *status and tells the team (`failed`, by the parity of the next barrier,
-// so that all four leave at the same one).
+// is drained (mbar_wait_drain), sets *status and tells the team (`failed`, by the
+// parity of the next barrier, so that all four leave at the same one).
 template <bool TRAIN>
 __global__ void __cluster_dims__(kTeam, 1, 1) __launch_bounds__(512, 1) mlp_rows_kernel(MlpRowsArgs a) {
     extern __shared__ unsigned char mraw[];
@@ -500,7 +517,7 @@ __global__ void __cluster_dims__(kTeam, 1, 1) __launch_bounds__(512, 1) mlp_rows
     auto product = [&](int q, int buf, bool forward, unsigned col, bool accumulate) {
         if (tid == 0) {
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            if (!mbar_wait_parity(&full[q % kRing], (unsigned)((q / kRing) & 1), kMlpPolls)) tell_failed();
+            if (!mbar_wait_drain(&full[q % kRing], (unsigned)((q / kRing) & 1), a.polls)) tell_failed();
             const __nv_bfloat16* A = act + buf * kBlk;
             const __nv_bfloat16* W = ring + (q % kRing) * kBlk;
 #pragma unroll
@@ -517,7 +534,7 @@ __global__ void __cluster_dims__(kTeam, 1, 1) __launch_bounds__(512, 1) mlp_rows
     };
     // product q is done; its weight block's slot is refilled
     auto finished = [&](int q) {
-        const bool ok = mbar_wait_parity(&mma_bar, (unsigned)(q & 1), kMlpPolls);
+        const bool ok = mbar_wait_drain(&mma_bar, (unsigned)(q & 1), a.polls);
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
         if (!ok) tell_failed();
         __syncthreads();
@@ -615,7 +632,7 @@ __global__ void __cluster_dims__(kTeam, 1, 1) __launch_bounds__(512, 1) mlp_rows
             if (NT > 2) {
                 if (tid == 0) {
                     blk_load(act + buf * kBlk, keep_dz + (size_t)(3 + nt) * kBlk, &rel_bar);
-                    if (!mbar_wait_parity(&rel_bar, (unsigned)(nt & 1), kMlpPolls)) tell_failed();
+                    if (!mbar_wait_drain(&rel_bar, (unsigned)(nt & 1), a.polls)) tell_failed();
                 }
                 __syncthreads();
             }
@@ -671,7 +688,7 @@ __global__ void __launch_bounds__(128, 1) mlp_dw_kernel(const __nv_bfloat16* __r
                                                         const __nv_bfloat16* __restrict__ dz,
                                                         const float* __restrict__ dzf, int KT, int NT, int nrb, int B,
                                                         float* __restrict__ grad, float* __restrict__ bgrad,
-                                                        int* __restrict__ status) {
+                                                        int* __restrict__ status, int polls) {
     extern __shared__ unsigned char mraw[];
     __shared__ __align__(8) unsigned long long full[kDwStages], read[kDwStages], done;
     __shared__ unsigned tmem_slot;
@@ -697,7 +714,7 @@ __global__ void __launch_bounds__(128, 1) mlp_dw_kernel(const __nv_bfloat16* __r
         bool ok = true;
         int i = 0;
         for (; ok && i < nrb; ++i) {
-            ok = __all_sync(0xffffffffu, mbar_wait_parity(&full[i % kDwStages], (unsigned)((i / kDwStages) & 1), kMlpPolls));
+            ok = __all_sync(0xffffffffu, mbar_wait_parity(&full[i % kDwStages], (unsigned)((i / kDwStages) & 1), polls));
             if (!ok) break;
             const float* d = (const float*)(buf + (size_t)(i % kDwStages) * kBiasStage) + lane;
             const int rows = min(128, B - i * 128);
@@ -753,27 +770,28 @@ __global__ void __launch_bounds__(128, 1) mlp_dw_kernel(const __nv_bfloat16* __r
         for (; loaded < nrb && loaded < kDwStages; ++loaded) load(loaded);
         for (; ok && used < nrb; ++used) {
             const int i = used;
-            ok = mbar_wait_parity(&full[i % kDwStages], (unsigned)((i / kDwStages) & 1), kMlpPolls);
+            ok = mbar_wait_parity(&full[i % kDwStages], (unsigned)((i / kDwStages) & 1), polls);
             if (!ok) break;
             const __nv_bfloat16* d = (const __nv_bfloat16*)(buf + (size_t)(i % kDwStages) * kDwStage);
             dw_mma(d, d + kBlk, tmem, i > 0);
             mma_commit(&read[i % kDwStages]);
             // the stage that the previous row block has left takes a new one
             if (i >= 1 && loaded < nrb) {
-                ok = mbar_wait_parity(&read[(i - 1) % kDwStages], (unsigned)(((i - 1) / kDwStages) & 1), kMlpPolls);
+                ok = mbar_wait_parity(&read[(i - 1) % kDwStages], (unsigned)(((i - 1) / kDwStages) & 1), polls);
                 if (ok) load(loaded++);
             }
         }
         if (!ok) {
-            atomicOr(status, 1);
             for (int j = used; j < loaded; ++j)  // no copy may land after the CTA ends
                 mbar_wait_parity(&full[j % kDwStages], (unsigned)((j / kDwStages) & 1), kMlpPolls);
         }
         mma_commit(&done);
     }
-    ok = mbar_wait_parity(&done, 0, kMlpPolls) && ok;
+    ok = mbar_wait_drain(&done, 0, polls) && ok;
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    if (!__syncthreads_or(!ok)) {
+    if (__syncthreads_or(!ok)) {
+        if (tid == 0) atomicOr(status, 1);
+    } else {
         // lane = output, tensor-memory column = input: each column is a coalesced row of the tile
         float* dst = grad + (size_t)tile * kBlk + (size_t)grp * 32 * 128 + warp * 32 + lane;
 #pragma unroll 1
@@ -851,7 +869,9 @@ __global__ void __launch_bounds__(256) mlp_update_kernel(MlpShape s, const float
                                                          const float* __restrict__ lossp, int nloss,
                                                          float* __restrict__ grads, float* __restrict__ w,
                                                          __nv_bfloat16* __restrict__ wp, float* __restrict__ m,
-                                                         float* __restrict__ v, float* __restrict__ loss, AdamArgs ad) {
+                                                         float* __restrict__ v, float* __restrict__ loss, AdamArgs ad,
+                                                         const int* __restrict__ status, int* __restrict__ skipped) {
+    if (update_skipped(status, skipped, ad.lr > 0.f)) return;
     const int tiles = s.KT + 2 + s.NT;
     if ((int)blockIdx.x < 8 * tiles) {
         const int tile = blockIdx.x >> 3;
@@ -926,10 +946,12 @@ struct edus_mlp {
     __nv_bfloat16* dzb = nullptr;
     float* loss = nullptr;
     int* status = nullptr;  // the word after loss: set when a bounded wait in a kernel ran out
+    int* skipped = nullptr; // the next word: training steps left out since (update_skipped)
     struct Report {
         float loss;
-        int status;
-    }* report = nullptr;    // pinned: loss and status of a step, read back in one copy
+        int status, skipped;
+    }* report = nullptr;    // pinned: the three words, read back in one copy
+    int polls = kMlpPolls;  // edus_mlp_set_wait_limit
     cudaStream_t stream = nullptr;
     // hidden width 128: weight blocks, and per 128-row block the operands of the weight gradients
     bool blocks = false;
@@ -965,8 +987,11 @@ int mlp_finish(edus_mlp* m, float* loss_host) {
     MCU(m, cudaStreamSynchronize(m->stream));
     if (loss_host) *loss_host = m->report->loss;
     if (m->report->status) {
-        MCU(m, cudaMemset(m->status, 0, sizeof(int)));
-        return mfail(m, EDUS_ERR_TIMEOUT, "a bounded wait for the tensor-core MMAs of a GEMM ran out");
+        m->step -= m->report->skipped;
+        MCU(m, cudaMemset(m->status, 0, 2 * sizeof(int)));
+        return mfail(m, EDUS_ERR_TIMEOUT,
+                     "a bounded wait of a network kernel ran out; training steps left out, weights as before them: " +
+                         std::to_string(m->report->skipped));
     }
     return EDUS_OK;
 }
@@ -1009,6 +1034,7 @@ MlpRowsArgs rows_args(edus_mlp* m, int B, const float* x, const float* t, float*
     a.lossp = m->lossp;
     a.scale = 1.f / (float)((long long)B * a.n_out);
     a.status = m->status;
+    a.polls = m->polls;
     return a;
 }
 
@@ -1019,10 +1045,10 @@ int blocks_backward(edus_mlp* m, int B, const float* x, const float* t, float lr
     const int nrb = (B + 127) / 128, tiles = m->shape.KT + 2 + m->shape.NT;
     mlp_rows_kernel<true><<<kTeam * nrb, 512, kRowsSmem, m->stream>>>(rows_args(m, B, x, t, nullptr));
     mlp_dw_kernel<<<dim3(tiles + 3 + m->shape.NT, 4), 128, kDwSmem, m->stream>>>(
-        m->actb, m->dzblk, m->dzf, m->shape.KT, m->shape.NT, nrb, B, m->dw, m->bgrad, m->status);
+        m->actb, m->dzblk, m->dzf, m->shape.KT, m->shape.NT, nrb, B, m->dw, m->bgrad, m->status, m->polls);
     mlp_update_kernel<<<8 * tiles + (384 + m->shape.n_out + 255) / 256 + 1, 256, 0, m->stream>>>(
         m->shape, m->dw, m->bgrad, m->lossp, kTeam * nrb, m->grads, m->params, m->wp, m->m, m->v, m->loss,
-        AdamArgs{lr, 0.9f, 0.999f, 1e-8f, c1, c2});
+        AdamArgs{lr, 0.9f, 0.999f, 1e-8f, c1, c2}, m->status, m->skipped);
     MCU(m, cudaGetLastError());
     return EDUS_OK;
 }
@@ -1031,7 +1057,7 @@ void gemm(edus_mlp* mm, int M, int N, int K, const __nv_bfloat16* A, long long a
           const __nv_bfloat16* B, long long b_rs, long long b_cs, float* C, int ldc, const float* bias) {
     dim3 grid((N + TN - 1) / TN, (M + TM - 1) / TM);
     gemm_bf16_kernel<<<grid, 128, 0, mm->stream>>>(M, N, K, A, a_rs, a_cs, B, b_rs, b_cs, C, ldc, bias, 0,
-                                                   mm->status);
+                                                   mm->status, mm->polls);
 }
 
 int ensure_cap(edus_mlp* m, int B) {
@@ -1152,6 +1178,7 @@ int edus_mlp_create(int n_in, int n_hidden, int n_out, unsigned long long seed, 
         return mfail(nullptr, EDUS_ERR_NOMEM, "MLP device allocation failed");
     }
     m->status = (int*)(m->loss + 1);
+    m->skipped = m->status + 1;
     // uniform initialisation scaled by the fan-in (seeded LCG), zero biases
     std::vector<float> p(off, 0.f);
     unsigned long long s = seed * 6364136223846793005ULL + 1442695040888963407ULL;
@@ -1210,8 +1237,15 @@ int edus_mlp_set_params(edus_mlp* m, const float* host) {
     else to_bf16_kernel<<<grid1(m->nparams), 256, 0, m->stream>>>(m->params, m->wbf, m->nparams);
     MCU(m, cudaMemsetAsync(m->m, 0, m->nparams * sizeof(float), m->stream));
     MCU(m, cudaMemsetAsync(m->v, 0, m->nparams * sizeof(float), m->stream));
+    MCU(m, cudaMemsetAsync(m->skipped, 0, sizeof(int), m->stream));  // steps before the new start
     m->step = 0;
     MCU(m, cudaStreamSynchronize(m->stream));
+    return EDUS_OK;
+}
+
+int edus_mlp_set_wait_limit(edus_mlp* m, int polls) {
+    if (!m) return EDUS_ERR_ARG;
+    m->polls = polls < 0 ? kMlpPolls : polls;
     return EDUS_OK;
 }
 
@@ -1219,8 +1253,7 @@ int edus_mlp_get_params(edus_mlp* m, float* host) {
     if (!m || !host) return EDUS_ERR_ARG;
     MCU(m, cudaSetDevice(m->device));
     MCU(m, cudaMemcpyAsync(host, m->params, m->nparams * sizeof(float), cudaMemcpyDeviceToHost, m->stream));
-    MCU(m, cudaStreamSynchronize(m->stream));
-    return EDUS_OK;
+    return mlp_finish(m, nullptr);
 }
 
 int edus_mlp_forward(edus_mlp* m, int batch, const float* x, float* y) {
@@ -1272,7 +1305,7 @@ int edus_mlp_train_step(edus_mlp* m, int batch, const float* x, const float* tar
         forward(m, batch, x);
         backward(m, batch, target);
         adam_kernel<<<grid1(m->nparams), 256, 0, m->stream>>>(m->params, m->wbf, m->grads, m->m, m->v, m->nparams, lr,
-                                                              b1, b2, 1e-8f, c1, c2);
+                                                              b1, b2, 1e-8f, c1, c2, m->status, m->skipped);
     }
     MCU(m, cudaGetLastError());
     return loss_host ? mlp_finish(m, loss_host) : EDUS_OK;

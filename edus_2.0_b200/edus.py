@@ -35,7 +35,8 @@ EXPORTS = [
     "edus_get_stream", "edus_set_profiling", "edus_get_profile", "edus_rhs_noalloc",
     "edus_set_anchor_interval", "edus_state_rspace", "edus_set_fock_override",
     "edus_mlp_create", "edus_mlp_destroy", "edus_mlp_last_error", "edus_mlp_param_count", "edus_mlp_set_params",
-    "edus_mlp_get_params", "edus_mlp_forward", "edus_mlp_gradients", "edus_mlp_train_step",    "edus_upload_model_solve", "edus_sweep_step", "edus_autotune",
+    "edus_mlp_get_params", "edus_mlp_forward", "edus_mlp_gradients", "edus_mlp_train_step", "edus_mlp_set_wait_limit",
+    "edus_upload_model_solve", "edus_sweep_step", "edus_autotune",
     "edus_upload_observables", "edus_observables", "edus_efield", "edus_set_kgradient",
     "edus_set_peierls", "edus_vector_potential", "edus_set_wait_limit",
 ]
@@ -137,6 +138,7 @@ def load_library(path: str | None = None):
     L.edus_mlp_forward.argtypes = [mp, ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p]
     L.edus_mlp_gradients.argtypes = [mp, ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p, fp, fp]
     L.edus_mlp_train_step.argtypes = [mp, ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_float, fp]
+    L.edus_mlp_set_wait_limit.argtypes = [mp, ctypes.c_int]
     L.edus_rhs_noalloc.argtypes = [P(ctypes.c_int), ctypes.c_int, ctypes.c_int, dp, dp, vp, vp, vp, vp, vp, vp, vp,
                                    vp, ctypes.c_char_p, ctypes.c_int]
     for name in EXPORTS:

@@ -110,6 +110,10 @@ class MLP:
                                                 loss.ctypes.data_as(ctypes.POINTER(ctypes.c_float))))
         return float(loss[0])
 
+    def set_wait_limit(self, polls: int):
+        """Poll limit of the kernels' bounded waits (negative: the default)."""
+        self._check(self._L.edus_mlp_set_wait_limit(self._h, int(polls)))
+
 
 def shell_indices(model, r_cut: float):
     """Natural R indices (j0 N1 + j1) N2 + j2 with |R| <= r_cut lattice vectors

@@ -252,6 +252,13 @@ int edus_mlp_gradients(edus_mlp* m, int batch, const float* x, const float* targ
                        float* loss_host);
 /* one Adam step on the batch; loss_host (may be NULL) receives the loss before the step */
 int edus_mlp_train_step(edus_mlp* m, int batch, const float* x, const float* target, float lr, float* loss_host);
+/* Poll limit of the network kernels' waits for their copies and tensor-core
+ * products (as edus_set_wait_limit: polls < 0 restores the default; 0 gives up
+ * without waiting, for exercising the failure path).  A wait that runs out is
+ * reported as EDUS_ERR_TIMEOUT by the next call that returns host data (a
+ * train_step with loss_host among them); until then training steps leave the
+ * weights, the optimiser's moments and the step count as they were. */
+int edus_mlp_set_wait_limit(edus_mlp* m, int polls);
 
 /* Split-precision form: steps between two moves of the anchor rho_ref to the
  * current state (>= 1; default 32).  No reference counterpart. */
