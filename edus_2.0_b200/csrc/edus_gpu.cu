@@ -186,8 +186,28 @@ int fail(edus_handle* h, int code, const std::string& msg) {
             return fail(h, EDUS_ERR_CUDA, std::string(#expr) + ": " + cudaGetErrorString(e_)); \
     } while (0)
 
-int dalloc(edus_handle* h, void** p, size_t bytes) {
+// cudaMalloc which, when memory is short, first gives back the one array a handle
+// can do without: H0 + E.xi of the TMA-fed commutator without HSEX (the handle
+// steps with the direct-load commutator from then on, as it would have without
+// room for the array in the first place).
+cudaError_t dev_malloc(edus_handle* h, void** p, size_t bytes) {
     cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaSuccess) cudaGetLastError();  // reported by the caller, not by the next launch's check
+    if (e == cudaErrorMemoryAllocation && h->ws_ipa && h->Hee && !h->peierls) {
+        cudaStreamSynchronize(h->stream);
+        h->allocs.erase(std::find(h->allocs.begin(), h->allocs.end(), (void*)h->Hee));
+        cudaFree(h->Hee);
+        h->Hee = nullptr;
+        h->ws_ipa = false;
+        h->dev_bytes -= h->S * h->B * sizeof(double2);
+        e = cudaMalloc(p, bytes);
+        if (e != cudaSuccess) cudaGetLastError();
+    }
+    return e;
+}
+
+int dalloc(edus_handle* h, void** p, size_t bytes) {
+    const cudaError_t e = dev_malloc(h, p, bytes);
     if (e != cudaSuccess) {
         *p = nullptr;
         return fail(h, EDUS_ERR_NOMEM, std::string("cudaMalloc(") + std::to_string(bytes) + "): " + cudaGetErrorString(e));
@@ -1015,7 +1035,7 @@ int build_sparse_model(edus_handle* h) {
     const int P = h->P, Nk = h->Nk;
     const size_t S = h->S;
     double2* tmp = nullptr;
-    CU(h, cudaMalloc((void**)&tmp, 4 * S * sizeof(double2)));
+    CU(h, dev_malloc(h, (void**)&tmp, 4 * S * sizeof(double2)));
     const double2* src[4] = {h->H0, h->xi[0], h->xi[1], h->xi[2]};
     for (int a = 0; a < 4; ++a)
         plane_to_R_kernel<kRadixAll, 256><<<P, 256, Nk * sizeof(double2), h->stream>>>(src[a], tmp + a * S, h->roots,
@@ -1606,7 +1626,6 @@ int edus_create(const edus_desc* desc, edus_handle** out) {
         TRY_ALLOC(h->rho0diag, h->nb * sizeof(double2));
         TRY_ALLOC(h->diag0, (size_t)h->B * h->nb * sizeof(double2));
     }
-    if (h->ws_ipa) TRY_ALLOC(h->Hee, SBb);
     TRY_ALLOC(h->roots, roots.size() * sizeof(double2));
     TRY_ALLOC(h->rpos, rpos.size() * sizeof(double));
     TRY_ALLOC(h->field, (size_t)h->chunk * 4 * h->B * sizeof(StageField));
@@ -1742,6 +1761,11 @@ int edus_create(const edus_desc* desc, edus_handle** out) {
         if ((rc = packed_setup_smem(h))) return bail(rc);
     }
 #undef TRY_ALLOC
+    // last, and optional: without room for it the direct-load commutator remains
+    if (h->ws_ipa && dalloc(h, (void**)&h->Hee, SBb) != EDUS_OK) {
+        h->ws_ipa = false;
+        h->err.clear();
+    }
     for (int i = 0; i < 2; ++i) {
         if (cudaMallocHost((void**)&h->field_host[i], (size_t)h->chunk * 4 * h->B * sizeof(StageField)) != cudaSuccess)
             return bail(fail(h, EDUS_ERR_NOMEM, "cudaMallocHost failed"));
@@ -2445,7 +2469,7 @@ static int fused_setup(edus_handle* const* hs, int n, int C, FusedSweep& f) {
             for (auto& x : *v) items.push_back(x.v);
     }
     auto alloc_copy = [&](void** p, const void* src, size_t bytes) -> int {
-        if (cudaMalloc(p, bytes) != cudaSuccess) return fail(h0, EDUS_ERR_CUDA, "fused sweep: cudaMalloc failed");
+        if (dev_malloc(h0, p, bytes) != cudaSuccess) return fail(h0, EDUS_ERR_CUDA, "fused sweep: cudaMalloc failed");
         if (src && cudaMemcpy(*p, src, bytes, cudaMemcpyHostToDevice) != cudaSuccess)
             return fail(h0, EDUS_ERR_CUDA, "fused sweep: upload failed");
         return EDUS_OK;
@@ -2836,7 +2860,7 @@ int edus_autotune(edus_handle* h, int* plane_threads, int* comm_tensor) {
         for (int c = 0; c < 3; ++c) x.g[c] = 1e-3 * (h->A[0 * 3 + c] + h->A[1 * 3 + c] + h->A[2 * 3 + c]);
     }
     StageField* df = nullptr;
-    CU(h, cudaMalloc((void**)&df, f.size() * sizeof(StageField)));
+    CU(h, dev_malloc(h, (void**)&df, f.size() * sizeof(StageField)));
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
@@ -2939,9 +2963,9 @@ int edus_state_rspace(edus_handle* h, int b, int nsel, const int* R_index, doubl
     double2* tmp = nullptr;
     int* dpos = nullptr;
     double2* dout = nullptr;
-    CU(h, cudaMalloc((void**)&tmp, h->S * sizeof(double2)));
-    if (cudaMalloc((void**)&dpos, nsel * sizeof(int)) != cudaSuccess ||
-        cudaMalloc((void**)&dout, (size_t)nsel * h->P * sizeof(double2)) != cudaSuccess) {
+    CU(h, dev_malloc(h, (void**)&tmp, h->S * sizeof(double2)));
+    if (dev_malloc(h, (void**)&dpos, nsel * sizeof(int)) != cudaSuccess ||
+        dev_malloc(h, (void**)&dout, (size_t)nsel * h->P * sizeof(double2)) != cudaSuccess) {
         cudaFree(tmp);
         cudaFree(dpos);
         return fail(h, EDUS_ERR_NOMEM, "edus_state_rspace: allocation failed");
