@@ -1069,10 +1069,8 @@ int build_sparse_model(edus_handle* h) {
         for (int p = 0; p < P; ++p)
             for (int s2 = 0; s2 < nS; ++s2) vals[((size_t)a * P + p) * nS + s2] = hv[a * S + (size_t)p * Nk + pos[s2]];
     int rc;
-    if (!h->hpos) {
-        if ((rc = dalloc(h, (void**)&h->hpos, kMaxSparseR * sizeof(int)))) return rc;
-        if ((rc = dalloc(h, (void**)&h->hval, 4 * (size_t)P * kMaxSparseR * sizeof(double2)))) return rc;
-    }
+    if (!h->hpos && (rc = dalloc(h, (void**)&h->hpos, kMaxSparseR * sizeof(int)))) return rc;
+    if (!h->hval && (rc = dalloc(h, (void**)&h->hval, 4 * (size_t)P * kMaxSparseR * sizeof(double2)))) return rc;
     CU(h, cudaMemcpyAsync(h->hpos, pos.data(), nS * sizeof(int), cudaMemcpyHostToDevice, h->stream));
     CU(h, cudaMemcpyAsync(h->hval, vals.data(), vals.size() * sizeof(double2), cudaMemcpyHostToDevice, h->stream));
     CU(h, cudaStreamSynchronize(h->stream));
@@ -1306,23 +1304,31 @@ int obs_grid(const edus_handle* h) { return h->nb <= 8 ? (h->Nk + 127) / 128 : s
 int obs_smem(const edus_handle* h) { return (int)(2 * h->P * sizeof(double2) + (2 * h->nb + 6 + 24) * sizeof(double)); }
 
 int ensure_obsacc(edus_handle* h) {
-    if (h->obsacc) return EDUS_OK;
+    if (h->obsacc) return EDUS_OK;  // the last of the two to be taken
     const size_t n = 2 * (size_t)h->nb + 6;
     int rc;
+    if (!h->obs_host && cudaMallocHost((void**)&h->obs_host, (n + 1) * sizeof(double)) != cudaSuccess) {
+        h->obs_host = nullptr;
+        cudaGetLastError();
+        return fail(h, EDUS_ERR_NOMEM, "cudaMallocHost failed");
+    }
     if ((rc = dalloc(h, (void**)&h->obsacc, (n + 1 + n * obs_grid(h) + 1) * sizeof(double)))) return rc;
     CU(h, cudaMemsetAsync(h->obsacc, 0, (n + 1 + n * obs_grid(h) + 1) * sizeof(double), h->stream));
-    if (cudaMallocHost((void**)&h->obs_host, (n + 1) * sizeof(double)) != cudaSuccess)
-        return fail(h, EDUS_ERR_NOMEM, "cudaMallocHost failed");
+    return EDUS_OK;
+}
+
+// The input and output planes of one right-hand side.
+int ensure_tmp(edus_handle* h) {
+    int rc;
+    if (!h->tmp_in && (rc = dalloc(h, (void**)&h->tmp_in, h->S * sizeof(double2)))) return rc;
+    if (!h->tmp_out && (rc = dalloc(h, (void**)&h->tmp_out, h->S * sizeof(double2)))) return rc;
     return EDUS_OK;
 }
 
 int fix_reference(edus_handle* h, int b) {
     int rc;
     const size_t Sb = h->S * sizeof(double2);
-    if (!h->tmp_in) {
-        if ((rc = dalloc(h, (void**)&h->tmp_in, Sb))) return rc;
-        if ((rc = dalloc(h, (void**)&h->tmp_out, Sb))) return rc;
-    }
+    if ((rc = ensure_tmp(h))) return rc;
     CU(h, cudaMemcpyAsync(h->ref_full, h->y + (size_t)b * h->S, Sb, cudaMemcpyDeviceToDevice, h->stream));
     StageField rf[4];
     for (int f = 0; f < 4; ++f) {
@@ -2060,7 +2066,7 @@ int edus_observables(edus_handle* h, int b, int filled, double* pop_bloch, doubl
     if (!h) return EDUS_ERR_ARG;
     if (b < 0 || b >= h->B) return fail(h, EDUS_ERR_ARG, "solve index out of range");
     if (pop_bloch && !h->obsU) return fail(h, EDUS_ERR_ARG, "the Bloch populations need edus_upload_observables(U)");
-    if (vel && !h->obsV[0]) return fail(h, EDUS_ERR_ARG, "the velocity needs edus_upload_observables(vel)");
+    if (vel && !h->obsV[2]) return fail(h, EDUS_ERR_ARG, "the velocity needs edus_upload_observables(vel)");
     int rc;
     CU(h, cudaSetDevice(h->d.device));
     if ((rc = ensure_obsacc(h))) return rc;
@@ -2127,9 +2133,9 @@ int edus_upload_model_solve(edus_handle* h, int b, const double* H0_k, const dou
     int rc;
     if (!h->per_solve) {
         // every solve starts from the shared model
-        if ((rc = dalloc(h, (void**)&h->H0b, Sb * h->B))) return rc;
+        if (!h->H0b && (rc = dalloc(h, (void**)&h->H0b, Sb * h->B))) return rc;
         for (int d = 0; d < 3; ++d)
-            if ((rc = dalloc(h, (void**)&h->xib[d], Sb * h->B))) return rc;
+            if (!h->xib[d] && (rc = dalloc(h, (void**)&h->xib[d], Sb * h->B))) return rc;
         for (int q = 0; q < h->B; ++q) {
             CU(h, cudaMemcpyAsync(h->H0b + (size_t)q * h->S, h->H0, Sb, cudaMemcpyDeviceToDevice, h->stream));
             for (int d = 0; d < 3; ++d)
@@ -2232,10 +2238,7 @@ int edus_rhs(edus_handle* h, double t, const double* in_k, double* out_k) {
         if ((rc0 = anchor_split(h))) return rc0;
     }
     int rc;
-    if (!h->tmp_in) {
-        if ((rc = dalloc(h, (void**)&h->tmp_in, h->S * sizeof(double2)))) return rc;
-        if ((rc = dalloc(h, (void**)&h->tmp_out, h->S * sizeof(double2)))) return rc;
-    }
+    if ((rc = ensure_tmp(h))) return rc;
     // field of solve 0 at time t, in slot 0 of the table (wait for the
     // previous user of the pinned buffer)
     CU(h, cudaEventSynchronize(h->field_ev[0]));

@@ -24,6 +24,7 @@ def hold_all_but():
         torch.cuda.synchronize()
         torch.cuda.empty_cache()
         held.append(torch.empty(torch.cuda.mem_get_info()[0] - n, dtype=torch.uint8, device="cuda"))
+        return held
 
     yield hold
     held.clear()
@@ -63,3 +64,42 @@ def test_optional_array_gives_way(pkg, po, tmp_path, hold_all_but, late):
         s = solver()
         assert s.device_bytes == full - STATE
     assert rel(run(s), ref) < 1e-13
+
+
+def test_sets_of_buffers_are_completed_by_the_next_call(pkg, po, tmp_path, hold_all_but):
+    """Buffers that serve together: when the allocation of the second fails, the
+    call reports it and the next one, with room again, takes what is missing."""
+    E = pkg.edus
+    cfg = po.load_input(model_input(pkg, tmp_path, "lowset", GRID, nb=NB, coulomb=True, dt=0.005, envelope="gauss"))
+    o = po.Oracle(cfg)
+    s = E.Solver(cfg.grid, NB, cfg.dt, coulomb=True)
+    s.upload_model(o.get("H0k"), np.stack([o.get("xk"), o.get("yk"), o.get("zk")]), o.lattice(), o.get("W"),
+                   o.get("DM0R"), o.hartree())
+    s.set_lasers(lasers_of(pkg, cfg))
+    s.set_state(o.get("rho"))
+    rho, one = o.get("rho"), STATE // BATCH
+
+    def release(held):
+        import torch
+
+        held.clear()
+        torch.cuda.empty_cache()
+
+    held = hold_all_but(one + one // 2)
+    vel = np.zeros((3,) + s.shape, dtype=complex)
+    with pytest.raises(E.EdusError) as ei:
+        s.upload_observables(vel=vel)  # room for one of its three arrays
+    assert ei.value.code == 6
+    s._has_vel = True  # the binding's own note of an upload: the library is asked
+    with pytest.raises(E.EdusError) as ei:
+        s.observables(0, 0)
+    assert ei.value.code == 1
+    release(held)
+    held = hold_all_but(one + one // 2)
+    with pytest.raises(E.EdusError) as ei:
+        s.rhs(3.0, rho)  # room for one of its two arrays
+    assert ei.value.code == 6
+    release(held)
+    assert rel(s.rhs(3.0, rho), o.rhs(3.0, rho)) < 1e-10
+    s.upload_observables(vel=vel)
+    assert np.array_equal(s.observables(0, 0)[2], np.zeros(3))
