@@ -33,6 +33,7 @@
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <cstdio>
 #include <mutex>
 #include <string>
@@ -42,6 +43,7 @@
 // this translation unit carries its own copies.
 namespace {
 #include "kernels.cuh"
+#include "launch_rules.hpp"
 #include "plane_plan.hpp"
 }  // namespace
 
@@ -245,8 +247,10 @@ extern "C" int edus_rhs_noalloc(const int grid[3], int nbands, int coulomb, cons
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return nfail(EDUS_ERR_CUDA, std::string("cudaGetDevice: ") + cudaGetErrorString(e));
     if (dev < 0 || dev >= kMaxDevices) return nfail(EDUS_ERR_UNSUPPORTED, "edus_rhs_noalloc: device ordinal too large");
-    int dev_smem = 0, sm_count = 0;
+    int dev_smem = 0, sm_count = 0, sm_smem = 0, cta_reserved = 0;
     cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
+    cudaDeviceGetAttribute(&sm_smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
+    cudaDeviceGetAttribute(&cta_reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev);
     cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     if (plane_smem > (size_t)dev_smem || comm_smem > (size_t)dev_smem)
         return nfail(EDUS_ERR_UNSUPPORTED, "edus_rhs_noalloc: k grid or band count too large for shared memory");
@@ -347,11 +351,8 @@ extern "C" int edus_rhs_noalloc(const int grid[3], int nbands, int coulomb, cons
     prep_inputs<<<dim3((Nk + 31) / 32, (P + 31) / 32, coulomb ? 3 : 2), tb, 0, stream>>>(pa);
     NA_CU(cudaGetLastError());
     dim3 pg(P, 1);
-    // More planes than SMs: 256 threads, so that two CTAs (128 registers a
-    // thread) share an SM and the planes run in one wave where they would take
-    // two (196 planes of 48 x 48 with HSEX: 50 -> 32 us); else 512 threads a plane.
     const bool wide = plane_launch(plan).variant == 2;  // radix 11 or 13
-    const int threads = P > sm_count ? 256 : 512;
+    const int threads = rhs_plane_threads(P, sm_count, plane_smem, (size_t)sm_smem, (size_t)cta_reserved);
     auto run_planes = [&](auto kernel) {
         kernel<<<pg, threads, plane_smem, stream>>>(rho_pk, 0, G, Hee, 0, r0p, Wp, diag0, d_field, d_roots, d_rpos, plan,
                                                     nb, 1.0 / Nk, nullptr, nullptr, 0, nullptr, 0);

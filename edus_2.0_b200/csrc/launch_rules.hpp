@@ -1,0 +1,17 @@
+// Which launch serves a call, by sizes alone (host code, no CUDA headers).
+#pragma once
+#include <cstddef>
+
+namespace edus {
+
+// Threads of a plane CTA in the device-buffer right-hand side.  With more planes
+// than SMs, 256, so that two CTAs (128 registers a thread) share an SM and the planes run
+// in one wave where they would take two: 196 planes of 48 x 48 with HSEX 50 -> 32 us.
+// A plane too large for two CTAs an SM has it to itself either way and keeps 512:
+// 169 plane pairs of 65 x 56, the whole call 147 us against 161 with 256.
+// (cta_reserved: what the system takes of an SM's shared memory for each CTA.)
+inline int rhs_plane_threads(int planes, int sms, size_t plane_smem, size_t sm_smem, size_t cta_reserved) {
+    return planes > sms && 2 * (plane_smem + cta_reserved) <= sm_smem ? 256 : 512;
+}
+
+}  // namespace edus
