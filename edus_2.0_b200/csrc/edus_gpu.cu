@@ -19,6 +19,7 @@
 #include "split_kernels.cuh"
 #include "plane3.cuh"
 #include "sweep_kernels.cuh"
+#include "launch_rules.hpp"
 #include "resident.cuh"
 #include <cudaTypedefs.h>
 #include <map>
@@ -68,7 +69,8 @@ struct edus_handle {
     // observables: eigenvectors U_k and velocity operator v_d(k), [P][Nk] each
     double2* obsU = nullptr;
     double2* obsV[3] = {nullptr, nullptr, nullptr};
-    double* obsacc = nullptr;      // sums and the status word, then the CTAs' partial sums and their counter
+    double* obsacc = nullptr;      // sums and the status word, then the CTAs' and the groups' sums and their counters
+    int obs_ctas = 0;
     double* obs_host = nullptr;    // pinned
     // a model (H0, xi) per solve (edus_upload_model_solve): [B][P][Nk] each
     bool per_solve = false;
@@ -1134,37 +1136,63 @@ __global__ void __launch_bounds__(MAXT) peierls_shift_kernel(const double2* __re
 // Observables: sums over k of the Bloch populations Re (U^dagger rho U)_nn
 // (values 0 .. nb - 1), the Wannier populations Re rho_nn (nb ..) and tr(v_d rho)
 // (2 nb ..: re, im of d = 0, 1, 2).
-// The CTAs' sums (fixed order: the result does not depend on which finishes
-// last) and the handle's status word into out, by the last CTA: part[cta][nacc].
-__device__ __forceinline__ void observables_finish(const double* mine, int nacc, double* __restrict__ part,
-                                                   double* __restrict__ out, const int* __restrict__ status,
-                                                   unsigned* __restrict__ count) {
-    for (int v = threadIdx.x; v < nacc; v += blockDim.x) part[(size_t)blockIdx.x * nacc + v] = mine[v];
-    __threadfence();
-    __syncthreads();
-    if (!__syncthreads_or(threadIdx.x == 0 && atomicAdd(count, 1u) == gridDim.x - 1)) return;
-    __threadfence();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int v = warp; v < nacc; v += blockDim.x >> 5) {
-        double s = 0.0;
-        for (int c = lane; c < (int)gridDim.x; c += 32) s += __ldcg(&part[(size_t)c * nacc + v]);
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == 0) out[v] = s;
+// The CTAs' sums, in a fixed order (the result does not depend on which CTA
+// finishes last): the last CTA of 32 adds the rows of those 32, the last of all
+// the rows so made, a thread a value with 16 loads in flight, and copies the
+// handle's status word.  One level over hundreds of CTAs was a chain of its own:
+// 32 bands on 24 x 24, 576 CTAs and 70 values, took 36 us longer than this.
+constexpr int kObsGroup = 32;
+__host__ __device__ inline int obs_groups(int ctas) { return (ctas + kObsGroup - 1) / kObsGroup; }
+struct ObsSums {
+    double *part, *gpart, *out;  // [cta][nacc], [group][nacc], [nacc + 1]
+    const int* status;
+    unsigned* count;             // [groups + 1], zero between launches
+};
+__device__ __forceinline__ void observables_finish(const double* mine, int nacc, const ObsSums& o) {
+    const int ctas = gridDim.x, groups = obs_groups(ctas), group = blockIdx.x / kObsGroup;
+    // add `rows` rows; true in the CTA that arrives last of `n` at `count`
+    auto add_rows = [&](const double* src, int rows, double* dst) {
+        for (int v = threadIdx.x; v < nacc; v += blockDim.x) {
+            double s = 0.0;
+            for (int c = 0; c < rows; c += 16) {
+                double x[16];
+#pragma unroll
+                for (int u = 0; u < 16; ++u) x[u] = c + u < rows ? __ldcg(&src[(size_t)(c + u) * nacc + v]) : 0.0;
+#pragma unroll
+                for (int u = 0; u < 16; ++u) s += x[u];
+            }
+            dst[v] = s;
+        }
+    };
+    auto last = [&](unsigned* count, int n) {
+        __threadfence();
+        __syncthreads();
+        const bool is = __syncthreads_or(threadIdx.x == 0 && atomicAdd(count, 1u) == (unsigned)n - 1u);
+        if (is) {
+            __threadfence();
+            if (threadIdx.x == 0) *count = 0;
+        }
+        return is;
+    };
+    for (int v = threadIdx.x; v < nacc; v += blockDim.x) o.part[(size_t)blockIdx.x * nacc + v] = mine[v];
+    const int first = group * kObsGroup, n = min(kObsGroup, ctas - first);
+    if (!last(&o.count[group], n)) return;
+    add_rows(o.part + (size_t)first * nacc, n, groups == 1 ? o.out : o.gpart + (size_t)group * nacc);
+    if (groups > 1) {
+        if (!last(&o.count[groups], groups)) return;
+        add_rows(o.gpart, groups, o.out);
     }
-    if (threadIdx.x == 0) {
-        out[nacc] = (double)*status;
-        *count = 0;
-    }
+    if (threadIdx.x == 0) o.out[nacc] = (double)*o.status;
 }
 
-// Few bands (nb <= 8): a thread per k point, planes read coalesced along k.
+// Few bands (obs_by_thread): a thread per k point, planes read coalesced along k.
 // One CTA per k point with an atomic per value (the general kernel's first form)
 // took 80 us for two bands on 50 x 50, all of it contention on ten words; 7 us here.
 __global__ void __launch_bounds__(128) observables_thread_kernel(
     const double2* __restrict__ rho, const double2* __restrict__ U, const double2* __restrict__ v0,
-    const double2* __restrict__ v1, const double2* __restrict__ v2, int Nk, int nb, double* __restrict__ part,
-    double* __restrict__ out, const int* __restrict__ status, unsigned* __restrict__ count) {
-    __shared__ double red[4][22], mine[22];
+    const double2* __restrict__ v1, const double2* __restrict__ v2, int Nk, int nb, ObsSums sums) {
+    constexpr int kValues = 2 * kObsThreadBands + 6;
+    __shared__ double red[4][kValues], mine[kValues];
     const int nacc = 2 * nb + 6, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int k = blockIdx.x * 128 + threadIdx.x;
     const bool on = k < Nk;
@@ -1199,15 +1227,16 @@ __global__ void __launch_bounds__(128) observables_thread_kernel(
     __syncthreads();
     for (int v = threadIdx.x; v < nacc; v += 128) mine[v] = red[0][v] + red[1][v] + red[2][v] + red[3][v];
     __syncthreads();
-    observables_finish(mine, nacc, part, out, status, count);
+    observables_finish(mine, nacc, sums);
 }
 
 // A CTA walks k points, rho_k and U_k in shared memory; its sums stay in
-// registers until the end.
+// registers until the end.  As many CTAs as the device holds at once: what bounds
+// them is a chain of nb^2 products a thread (592 CTAs, four an SM, took 263 us a
+// call for 22 bands on 72 x 72; this many, 180).
 __global__ void __launch_bounds__(128) observables_kernel(
     const double2* __restrict__ rho, const double2* __restrict__ U, const double2* __restrict__ v0,
-    const double2* __restrict__ v1, const double2* __restrict__ v2, int Nk, int nb, double* __restrict__ part,
-    double* __restrict__ out, const int* __restrict__ status, unsigned* __restrict__ count) {
+    const double2* __restrict__ v1, const double2* __restrict__ v2, int Nk, int nb, ObsSums sums) {
     extern __shared__ double2 so[];
     const int P = nb * nb, nacc = 2 * nb + 6;
     double2* R = so;
@@ -1261,7 +1290,7 @@ __global__ void __launch_bounds__(128) observables_kernel(
     if (threadIdx.x < 6)
         mine[2 * nb + threadIdx.x] = red[0][threadIdx.x] + red[1][threadIdx.x] + red[2][threadIdx.x] + red[3][threadIdx.x];
     __syncthreads();
-    observables_finish(mine, nacc, part, out, status, count);
+    observables_finish(mine, nacc, sums);
 }
 
 // plane position (digit-reversed order) of the natural R index (j0 N1 + j1) N2 + j2
@@ -1297,23 +1326,29 @@ int check_status(edus_handle* h) {
     return EDUS_OK;
 }
 
-// CTAs of the observables kernel
-int obs_grid(const edus_handle* h) { return h->nb <= 8 ? (h->Nk + 127) / 128 : std::min(h->Nk, 592); }
-
-// and its shared memory: rho_k, U_k, the sums and the warps' velocity sums
+// shared memory of observables_kernel: rho_k, U_k, the sums and the warps' velocity sums
 int obs_smem(const edus_handle* h) { return (int)(2 * h->P * sizeof(double2) + (2 * h->nb + 6 + 24) * sizeof(double)); }
 
 int ensure_obsacc(edus_handle* h) {
     if (h->obsacc) return EDUS_OK;  // the last of the two to be taken
-    const size_t n = 2 * (size_t)h->nb + 6;
+    if (obs_by_thread(h->nb)) {
+        h->obs_ctas = (h->Nk + 127) / 128;
+    } else {
+        int nsm = 0, per_sm = 0;
+        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->d.device);
+        CU(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, observables_kernel, 128, obs_smem(h)));
+        h->obs_ctas = std::min(h->Nk, std::max(1, per_sm) * std::max(1, nsm));
+    }
+    const size_t n = 2 * (size_t)h->nb + 6, groups = obs_groups(h->obs_ctas);
+    const size_t bytes = (n + 1 + n * (h->obs_ctas + groups)) * sizeof(double) + (groups + 1) * sizeof(unsigned);
     int rc;
     if (!h->obs_host && cudaMallocHost((void**)&h->obs_host, (n + 1) * sizeof(double)) != cudaSuccess) {
         h->obs_host = nullptr;
         cudaGetLastError();
         return fail(h, EDUS_ERR_NOMEM, "cudaMallocHost failed");
     }
-    if ((rc = dalloc(h, (void**)&h->obsacc, (n + 1 + n * obs_grid(h) + 1) * sizeof(double)))) return rc;
-    CU(h, cudaMemsetAsync(h->obsacc, 0, (n + 1 + n * obs_grid(h) + 1) * sizeof(double), h->stream));
+    if ((rc = dalloc(h, (void**)&h->obsacc, bytes))) return rc;
+    CU(h, cudaMemsetAsync(h->obsacc, 0, bytes, h->stream));
     return EDUS_OK;
 }
 
@@ -2086,16 +2121,18 @@ int edus_observables(edus_handle* h, int b, int filled, double* pop_bloch, doubl
         CU(h, cudaGetLastError());
         rho = h->stage;
     }
-    double* part = h->obsacc + nacc + 1;
-    unsigned* count = (unsigned*)(part + (size_t)nacc * obs_grid(h));
-    if (h->nb <= 8)
-        observables_thread_kernel<<<obs_grid(h), 128, 0, h->stream>>>(rho, pop_bloch ? h->obsU : nullptr,
-                                                                      vel ? h->obsV[0] : nullptr, h->obsV[1], h->obsV[2],
-                                                                      h->Nk, h->nb, part, h->obsacc, h->flag, count);
+    ObsSums sums{};
+    sums.out = h->obsacc;
+    sums.part = h->obsacc + nacc + 1;
+    sums.gpart = sums.part + (size_t)nacc * h->obs_ctas;
+    sums.count = (unsigned*)(sums.gpart + (size_t)nacc * obs_groups(h->obs_ctas));
+    sums.status = h->flag;
+    if (obs_by_thread(h->nb))
+        observables_thread_kernel<<<h->obs_ctas, 128, 0, h->stream>>>(
+            rho, pop_bloch ? h->obsU : nullptr, vel ? h->obsV[0] : nullptr, h->obsV[1], h->obsV[2], h->Nk, h->nb, sums);
     else
-        observables_kernel<<<obs_grid(h), 128, obs_smem(h), h->stream>>>(
-            rho, pop_bloch ? h->obsU : nullptr, vel ? h->obsV[0] : nullptr, h->obsV[1], h->obsV[2], h->Nk, h->nb, part,
-            h->obsacc, h->flag, count);
+        observables_kernel<<<h->obs_ctas, 128, obs_smem(h), h->stream>>>(
+            rho, pop_bloch ? h->obsU : nullptr, vel ? h->obsV[0] : nullptr, h->obsV[1], h->obsV[2], h->Nk, h->nb, sums);
     h->launches++;
     CU(h, cudaGetLastError());
     // the sums and the status word in one copy

@@ -14,4 +14,14 @@ inline int rhs_plane_threads(int planes, int sms, size_t plane_smem, size_t sm_s
     return planes > sms && 2 * (plane_smem + cta_reserved) <= sm_smem ? 256 : 512;
 }
 
+// Observables: a thread per k point (few bands) or a CTA per k point.  A thread
+// does nb^3 dependent products whatever the grid, a CTA spreads them: with
+// velocities and populations, a call of 4 bands takes 50 us against 49 (24 x 24) and
+// 52 against 68 (120 x 120), of 5 bands 62 against 49 and 64 against 75, of 8 bands
+// 86 against 47 and 96 against 99.  Up to four bands the thread never loses by more
+// than the two calls' spread; from five on the CTA is what is never slower than
+// the form before both (an atomic a value from every k point).
+constexpr int kObsThreadBands = 4;
+inline bool obs_by_thread(int nb) { return nb <= kObsThreadBands; }
+
 }  // namespace edus

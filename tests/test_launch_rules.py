@@ -15,6 +15,9 @@ CHECKS = {
     "rhs_plane_threads(169, 148, 115712, 233472, 1024)": 256,
     "rhs_plane_threads(169, 148, 115713, 233472, 1024)": 512,
     "rhs_plane_threads(169, 148, 2 * 65 * 56 * 16, 233472, 1024)": 512,
+    "obs_by_thread(1)": 1,
+    "obs_by_thread(4)": 1,
+    "obs_by_thread(5)": 0,
 }
 
 
