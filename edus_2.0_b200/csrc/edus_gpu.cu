@@ -858,6 +858,11 @@ double resident_cycles(const edus_handle* h, const ResidentGeom& g) {
             const double pts = d == 0 ? cols : rows;
             cyc += (rounds(pts / r) + rounds(pts * (c ? 2 : 1) / r)) * (500.0 + 100.0 * r);
         }
+    // The last stage of the unit-stride axis reads and writes runs of its radix:
+    // 16-byte elements meet in the banks as many ways as the radix divides by 2 (64
+    // points: two radices 8, 8 ways).  Counted where a stage is long enough for it to
+    // decide (3 bands on 64 x 64: 17.0 us without this, 20.2 with, 19.9 measured).
+    if (h->use3) cyc += rows / 8 * (gcd_int(h->plan.ax[1].r[h->plan.ax[1].nst - 1], 8) - 1) * (c ? 5 : 3);
     const int half = (h->nb + 1) / 2;
     cyc += rounds((double)half * half * rows / h->P) * (1500.0 + 450.0 * h->nb);
     cyc += 0.5 * rounds(rows / 4) * 5000.0;
@@ -881,10 +886,7 @@ int resident_setup(edus_handle* h) {
             h->res = g;
         }
     }
-    // The launches per stage instead: two kernels (four where planes are spread
-    // over many CTAs) of 4.5-5 us each when nothing but latency counts, and ten
-    // array passes over the solves' states at about 2 TB/s.
-    const double launches_us = (h->use3 ? 20.0 : 9.0) + 160.0 * (double)h->S * h->B / 2.0e6;
+    const double launches_us = staged_stage_us(h->use3, c, rk, (double)h->S * h->B);
     const double own_us = 1.2 * best / 1900.0;  // a margin of 20% to the estimate
     if (own_us >= launches_us) return EDUS_OK;
     int rc;

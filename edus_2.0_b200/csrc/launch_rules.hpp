@@ -14,6 +14,18 @@ inline int rhs_plane_threads(int planes, int sms, size_t plane_smem, size_t sm_s
     return planes > sms && 2 * (plane_smem + cta_reserved) <= sm_smem ? 256 : 512;
 }
 
+// Estimated microseconds of a stage in launches, for problems where nothing but
+// latency counts: the launches and ten passes over the solves' states (`elements`)
+// at about 2 TB/s.  Two launches take 9 us at the least.  Where planes are spread over
+// many CTAs there are four: measured 17 to 19 us replayed from a CUDA graph (RK4, long
+// calls) and 24 to 27 launched, with HSEX 25 to 27 and 33 to 35; Adams-Bashforth has
+// no graphs.  The choice must not depend on a call's length, or a split call would
+// round differently, so RK4 counts near its replayed time.
+inline double staged_stage_us(bool spread, bool hsex, bool rk, double elements) {
+    const double launches = !spread ? 9.0 : (hsex ? 26.0 : 20.0) + (rk ? 0.0 : 4.0);
+    return launches + 160.0 * elements / 2.0e6;
+}
+
 // Observables: a thread per k point (few bands) or a CTA per k point.  A thread
 // does nb^3 dependent products whatever the grid, a CTA spreads them: with
 // velocities and populations, a call of 4 bands takes 50 us against 49 (24 x 24) and

@@ -15,6 +15,11 @@ CHECKS = {
     "rhs_plane_threads(169, 148, 115712, 233472, 1024)": 256,
     "rhs_plane_threads(169, 148, 115713, 233472, 1024)": 512,
     "rhs_plane_threads(169, 148, 2 * 65 * 56 * 16, 233472, 1024)": 512,
+    "staged_stage_us(false, false, true, 0)": 9,
+    "staged_stage_us(false, true, false, 1e5)": 17,
+    "staged_stage_us(true, false, true, 0)": 20,
+    "staged_stage_us(true, true, true, 0)": 26,
+    "staged_stage_us(true, false, false, 0)": 24,
     "obs_by_thread(1)": 1,
     "obs_by_thread(4)": 1,
     "obs_by_thread(5)": 0,
