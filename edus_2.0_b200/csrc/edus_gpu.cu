@@ -87,8 +87,8 @@ struct edus_handle {
     // box kind): kind 0 the dense box, kind 1 the zero-padded box of the
     // product operands
     bool comm_ws = false;
-    // the same kernel without HSEX, for states too large for L2: H0 + E.xi is
-    // written to Hee when E changes (hamiltonian_kernel)
+    // the same kernel without HSEX (ws_ipa_bytes): H0 + E.xi is written to Hee when
+    // E changes (hamiltonian_kernel)
     bool ws_ipa = false;
     const StageField* prev_field = nullptr;  // field of the stage launched before, when Hee holds its H
     int ws_grid = 0;
@@ -1603,9 +1603,8 @@ int edus_create(const edus_desc* desc, edus_handle** out) {
     if ((rc = set_smem(h, commutator_mma_kernel<M, false, true>, smem_cmax))) return bail(rc);
     SETC(MODE_RHS) SETC(MODE_RK1) SETC(MODE_RK2) SETC(MODE_RK3) SETC(MODE_RK4) SETC(MODE_AB)
 #undef SETC
-    // Without HSEX from 12 MB of state (all solves) up: below, the extra launch
-    // that writes H0 + E.xi costs as much as the tiles it relieves.
-    const bool want_ws_ipa = !d.coulomb && d.precision == EDUS_PREC_FP64 && h->S * h->B * sizeof(double2) >= (12u << 20);
+    const bool want_ws_ipa = !d.coulomb && d.precision == EDUS_PREC_FP64 &&
+                             h->S * h->B * sizeof(double2) >= ws_ipa_bytes(h->nb, d.solver == EDUS_SOLVER_AB);
     if ((d.coulomb || want_ws_ipa) && ws_supported(h->nb) && tensor_map_encoder()) {
         const WsGeom wg = ws_geometry(h->nb);
         if ((int)wg.smem <= dev_smem) {

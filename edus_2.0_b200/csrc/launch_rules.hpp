@@ -26,6 +26,14 @@ inline double staged_stage_us(bool spread, bool hsex, bool rk, double elements) 
     return launches + 160.0 * elements / 2.0e6;
 }
 
+// State (all solves) from which the TMA-fed commutator serves without HSEX.  Below,
+// the launch that writes H0 + E.xi costs as much as the tiles it relieves: RK4 from
+// 12 MB gains 6 to 26% over 12 to 24 bands.  Adams-Bashforth writes H every step
+// instead of twice in four stages, and 16 bands fill the direct-load kernel's 8 x 8
+// tiles: 28 x 28, four solves (12.2 MB) 82 -> 87 us a step, and even or faster from
+// 14 MB (64 x 64, 16 MB: 105 -> 98; 15 bands, 63 x 60, 13 MB: 87 -> 81).
+inline size_t ws_ipa_bytes(int nb, bool adams) { return (size_t)(adams && nb == 16 ? 14 : 12) << 20; }
+
 // Observables: a thread per k point (few bands) or a CTA per k point.  A thread
 // does nb^3 dependent products whatever the grid, a CTA spreads them: with
 // velocities and populations, a call of 4 bands takes 50 us against 49 (24 x 24) and

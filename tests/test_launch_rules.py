@@ -20,6 +20,11 @@ CHECKS = {
     "staged_stage_us(true, false, true, 0)": 20,
     "staged_stage_us(true, true, true, 0)": 26,
     "staged_stage_us(true, false, false, 0)": 24,
+    "(double)ws_ipa_bytes(12, false)": 12 << 20,
+    "(double)ws_ipa_bytes(16, false)": 12 << 20,
+    "(double)ws_ipa_bytes(15, true)": 12 << 20,
+    "(double)ws_ipa_bytes(16, true)": 14 << 20,
+    "(double)ws_ipa_bytes(17, true)": 12 << 20,
     "obs_by_thread(1)": 1,
     "obs_by_thread(4)": 1,
     "obs_by_thread(5)": 0,
@@ -34,7 +39,7 @@ def rules(tmp_path_factory):
     d = tmp_path_factory.mktemp("rules")
     src = d / "rules.cpp"
     src.write_text('#include <cstdio>\n#include "launch_rules.hpp"\nusing namespace edus;\nint main() {\n'
-                   + "".join(f'    std::printf("%g\\n", (double)({c}));\n' for c in CHECKS) + "}\n")
+                   + "".join(f'    std::printf("%.17g\\n", (double)({c}));\n' for c in CHECKS) + "}\n")
     subprocess.run([gxx, "-std=c++17", "-Wall", "-Werror", "-I", os.path.join(ROOT, "edus_2.0_b200", "csrc"), str(src),
                     "-o", str(d / "rules")], check=True)
     out = subprocess.run([str(d / "rules")], check=True, capture_output=True, text=True).stdout.split()
