@@ -2762,10 +2762,14 @@ int edus_sweep_step(edus_handle* const* hs, int n, int steps, int use_graph) {
     cudaGraphExec_t exec = nullptr;
     FusedSweep fs;
     int rc = EDUS_OK;
-    // the fused launches take the handles that do not step by the resident
-    // kernel; those that do run beside them, each on its own stream
+    // The fused launches take the handles that would step with the same kernels
+    // alone.  Those that step in one launch, or with the TMA-fed commutator, run beside
+    // them, each on its own stream: every result equals stepping the handle alone, and
+    // large states are faster so (two solves of 22 bands 96x96 among four smaller shapes:
+    // 4080 -> 3451 us a step; 22 bands 72x72 and eight solves of 2 bands: 848 -> 566).
     std::vector<edus_handle*> hf, hown;
-    for (int i = 0; i < n; ++i) (fused && !resident_active(hs[i]) ? hf : hown).push_back(hs[i]);
+    for (int i = 0; i < n; ++i)
+        (fused && !resident_active(hs[i]) && !hs[i]->ws_ipa ? hf : hown).push_back(hs[i]);
     std::vector<unsigned long long> chunk_launches(n, 0);
     auto cleanup = [&]() {
         if (s0) cudaStreamSynchronize(s0);

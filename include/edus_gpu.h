@@ -207,10 +207,11 @@ int edus_step(edus_handle* h, int n);
  *                  chunks captured into a CUDA graph.  RK4, independent
  *                  particles, R-space gradient, length gauge (else
  *                  EDUS_ERR_UNSUPPORTED).  Handles that step in one launch of
- *                  their own (edus_step) run beside the fused launches.
+ *                  their own (edus_step), and large states (12 to 24 bands
+ *                  from 12 MB), run beside the fused launches.
  * A solve's result equals stepping its handle alone (in the fused form to
- * rounding, where the handle alone takes other kernels: many CTAs a plane, or
- * the TMA-fed commutator of large states).
+ * rounding, where the handle alone spreads each plane over many CTAs: grids of
+ * 1024 points and more with fewer planes than SMs).
  * Synchronous.  No reference counterpart. */
 int edus_sweep_step(edus_handle* const* hs, int n, int steps, int use_graph);
 
