@@ -2442,9 +2442,6 @@ static bool fused_eligible(const edus_handle* h) {
 
 static int fused_setup(edus_handle* const* hs, int n, int C, FusedSweep& f) {
     edus_handle* h0 = hs[0];
-    if (n > kSweepMaxShapes)
-        return fail(h0, EDUS_ERR_UNSUPPORTED,
-                    "the fused sweep takes at most " + std::to_string(kSweepMaxShapes) + " handles");
     f.n = n;
     f.C = C;
     std::vector<PlanePlan> plans(n);
@@ -2754,6 +2751,10 @@ int edus_sweep_step(edus_handle* const* hs, int n, int steps, int use_graph) {
                         "or profiling)");
     }
     if (steps == 0) return EDUS_OK;
+    // of all handles, fused or beside: what is accepted does not hang on how each would step
+    if (fused && n > kSweepMaxShapes)
+        return fail(h0, EDUS_ERR_UNSUPPORTED,
+                    "the fused sweep takes at most " + std::to_string(kSweepMaxShapes) + " handles");
     CU(h0, cudaSetDevice(h0->d.device));
     constexpr int C = 32;  // steps per captured chunk (<= the field-table capacity)
     cudaStream_t s0 = nullptr;

@@ -45,3 +45,19 @@ def test_large_states_step_as_alone(pkg, po, tmp_path, steps):
     sweep as alone, beside a fused shape."""
     pairs = make(pkg, po, tmp_path, [(22, (48, 48, 1), 2), (7, (36, 36, 1), 4)])
     check(pkg, pairs, steps, [12 * steps, 8 * steps], fused=True)
+
+
+def test_handle_limit_counts_every_handle(pkg):
+    """More than 64 handles are refused, however they would step (these: each in one launch)."""
+    E = pkg.edus
+    H = np.zeros((16, 2, 2), dtype=complex)
+    ss = []
+    for _ in range(65):
+        s = E.Solver((4, 4, 1), 2, 0.05)
+        s.upload_model(H, np.stack([H] * 3), np.eye(3))
+        ss.append(s)
+    with pytest.raises(E.EdusError) as ei:
+        E.sweep_step(ss, 2, fused=True)
+    assert ei.value.code == 5 and ss[0].time == 0.0
+    E.sweep_step(ss[:64], 2, fused=True)
+    assert ss[0].time == 0.1
