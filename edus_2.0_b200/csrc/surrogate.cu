@@ -266,9 +266,11 @@ __global__ void adam_kernel(float* __restrict__ w, __nv_bfloat16* __restrict__ w
 }
 
 // ---------------------------------------------------------------------------
-// Networks of hidden width 128 (what the surrogate uses): the whole forward
-// and backward chain of 128 batch rows in one CTA, the weight gradients in one
-// grouped split-K launch, reduction and Adam in a third.
+// Networks of hidden width 128 (what the surrogate uses; other widths run the
+// kernels above): the whole forward and backward chain of 128 batch rows in a
+// cluster of four CTAs, all weight and bias gradients in a second launch (each a
+// contraction over the whole batch, not split), Adam and the weights' BF16 blocks in
+// a third.
 //
 // Layer by layer through global memory this step was bound by its launches and
 // by serial work, not by arithmetic: the weight gradients contract over the
@@ -933,7 +935,7 @@ struct edus_mlp {
     float* grads = nullptr;
     float* m = nullptr;
     float* v = nullptr;
-    __nv_bfloat16* wbf = nullptr;  // BF16 copy (same offsets as params)
+    __nv_bfloat16* wbf = nullptr;  // BF16 copy (same offsets as params); the 128-wide form has wp instead
     long long woff[kLayers] = {0}, boff[kLayers] = {0};
     int step = 0;
     // activations for a batch of up to `cap` samples
@@ -1170,7 +1172,7 @@ int edus_mlp_create(int n_in, int n_hidden, int n_out, unsigned long long seed, 
         cudaMalloc((void**)&m->grads, off * sizeof(float)) != cudaSuccess ||
         cudaMalloc((void**)&m->m, off * sizeof(float)) != cudaSuccess ||
         cudaMalloc((void**)&m->v, off * sizeof(float)) != cudaSuccess ||
-        cudaMalloc((void**)&m->wbf, off * sizeof(__nv_bfloat16)) != cudaSuccess ||
+        (!m->blocks && cudaMalloc((void**)&m->wbf, off * sizeof(__nv_bfloat16)) != cudaSuccess) ||
         cudaMalloc((void**)&m->loss, sizeof(*m->report)) != cudaSuccess ||
         cudaMallocHost((void**)&m->report, sizeof(*m->report)) != cudaSuccess ||
         cudaMemset(m->loss, 0, sizeof(*m->report)) != cudaSuccess) {

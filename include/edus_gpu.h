@@ -236,7 +236,11 @@ int edus_set_fock_override(edus_handle* h, int nsel, const int* R_index, const d
 
 /* Learned self-energy network: a multilayer perceptron n_in -> 3 hidden layers
  * of n_hidden (GELU) -> n_out, BF16 weights with FP32 master copies and FP32
- * accumulation, trained on the GPU (mean squared error, Adam).  Batches are
+ * accumulation, trained on the GPU (mean squared error, Adam).  n_hidden = 128
+ * (the package's default) has kernels of its own: three launches a training step;
+ * other widths go layer by layer, about 30 times slower (4096 rows, 259 -> 254:
+ * 4 ms a step against 0.12).  The first call with more rows than before
+ * allocates its workspace.  Batches are
  * row-major [batch][features] FP32 DEVICE buffers.  Parameters are flattened
  * as W0 b0 W1 b1 W2 b2 W3 b3, W_l row-major [in][out] (host FP32 buffers).
  * No reference counterpart. */
@@ -331,7 +335,9 @@ int edus_set_wait_limit(edus_handle* h, int polls);
 /* Per-kernel timing with CUDA events on the handle's stream (off by default).
  * kind 0 = plane kernel (k<->R transforms + gradient + HSEX), 1 = commutator
  * + stage kernel.  Totals accumulate from the call that enabled profiling;
- * edus_get_profile synchronises the stream. */
+ * edus_get_profile synchronises the stream.  A handle that steps in one launch
+ * (edus_step) has no such kernels; while profiled it steps by launches per
+ * stage, and the times are theirs. */
 int edus_set_profiling(edus_handle* h, int on);
 int edus_get_profile(edus_handle* h, int kind, double* total_ms, unsigned long long* launches);
 
