@@ -1140,7 +1140,8 @@ __global__ void __launch_bounds__(MAXT) peierls_shift_kernel(const double2* __re
 // (2 nb ..: re, im of d = 0, 1, 2).
 // The CTAs' sums, in a fixed order (the result does not depend on which CTA
 // finishes last): the last CTA of 32 adds the rows of those 32, the last of all
-// the rows so made, a thread a value with 16 loads in flight, and copies the
+// the rows so made, a thread a value, 16 loads in flight, added pairwise (in a row
+// they would round more: 2.4e-14 for 2.0e-14 over 20 CTAs), and copies the
 // handle's status word.  One level over hundreds of CTAs was a chain of its own:
 // 32 bands on 24 x 24, 576 CTAs and 70 values, took 36 us longer than this.
 constexpr int kObsGroup = 32;
@@ -1152,20 +1153,27 @@ struct ObsSums {
 };
 __device__ __forceinline__ void observables_finish(const double* mine, int nacc, const ObsSums& o) {
     const int ctas = gridDim.x, groups = obs_groups(ctas), group = blockIdx.x / kObsGroup;
-    // add `rows` rows; true in the CTA that arrives last of `n` at `count`
+    // `rows` rows into dst
     auto add_rows = [&](const double* src, int rows, double* dst) {
         for (int v = threadIdx.x; v < nacc; v += blockDim.x) {
             double s = 0.0;
-            for (int c = 0; c < rows; c += 16) {
+            auto at = [&](int c) { return c < rows ? __ldcg(&src[(size_t)c * nacc + v]) : 0.0; };
+            for (int c = 0; c < rows; c += 32) {
                 double x[16];
 #pragma unroll
-                for (int u = 0; u < 16; ++u) x[u] = c + u < rows ? __ldcg(&src[(size_t)(c + u) * nacc + v]) : 0.0;
+                for (int u = 0; u < 16; ++u) x[u] = at(c + u);
 #pragma unroll
-                for (int u = 0; u < 16; ++u) s += x[u];
+                for (int u = 0; u < 16; ++u) x[u] += at(c + 16 + u);
+#pragma unroll
+                for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+                    for (int u = 0; u < o; ++u) x[u] += x[u + o];
+                s += x[0];
             }
             dst[v] = s;
         }
     };
+    // true in the CTA that arrives last of `n` at `count`
     auto last = [&](unsigned* count, int n) {
         __threadfence();
         __syncthreads();
@@ -1235,8 +1243,9 @@ __global__ void __launch_bounds__(128) observables_thread_kernel(
 // A CTA walks k points, rho_k and U_k in shared memory; its sums stay in
 // registers until the end.  As many CTAs as the device holds at once: what bounds
 // them is a chain of nb^2 products a thread (592 CTAs, four an SM, took 263 us a
-// call for 22 bands on 72 x 72; this many, 180).
-__global__ void __launch_bounds__(128) observables_kernel(
+// call for 22 bands on 72 x 72; six an SM, at 80 registers, 183; five, where the
+// sums at the end set the register count, 244).
+__global__ void __launch_bounds__(128, 6) observables_kernel(
     const double2* __restrict__ rho, const double2* __restrict__ U, const double2* __restrict__ v0,
     const double2* __restrict__ v1, const double2* __restrict__ v2, int Nk, int nb, ObsSums sums) {
     extern __shared__ double2 so[];

@@ -31,3 +31,21 @@ def test_observables_against_numpy(pkg, tmp_path, nb, grid):
     for got, ref in zip(first, (bl, wn, v)):
         assert np.abs(got - ref).max() < 1e-12 * max(1.0, np.abs(ref).max())
     assert all(np.array_equal(a, b) for a, b in zip(first, s.observables(0, 0)))
+
+
+def test_sums_round_no_more_than_pairwise(pkg):
+    """Wannier populations are sums of Nk given numbers: the CTAs' sums (20 on 50 x 50) are added
+    pairwise, and so are the warps' lanes, so the error stays below 16 units of 2^-53 of
+    the sum of magnitudes (about log2 of the 2500 terms, and 4 more for the CTA's warps)."""
+    import math
+
+    s = pkg.edus.Solver((50, 50, 1), 2, 0.05)
+    H = np.zeros(s.shape, dtype=complex)
+    s.upload_model(H, np.stack([H] * 3), np.eye(3) * 6.0)
+    rng = np.random.default_rng(3)
+    rho = rng.uniform(0.1, 1.0, s.shape).astype(complex)
+    s.set_state(rho)
+    wn = s.observables(0, 0)[1]
+    for n in range(2):
+        exact = math.fsum(rho[:, n, n].real) / 2500
+        assert abs(wn[n] - exact) <= 16 * 2.0 ** -53 * exact
