@@ -242,8 +242,9 @@ __global__ void colsum_kernel(const float* __restrict__ dz, float* __restrict__ 
 // that made its gradients (or in an earlier step's, not reported yet): status
 // stays set until the host reads it, and `skipped` counts the training steps
 // that were left out, which the host takes back from its step count.
-__device__ __forceinline__ bool update_skipped(const int* status, int* skipped, bool training) {
-    if (!*status) return false;
+// `status` is read beside the operands, which the kernel waits for anyway.
+__device__ __forceinline__ bool update_skipped(int status, int* skipped, bool training) {
+    if (!status) return false;
     if (training && blockIdx.x == 0 && threadIdx.x == 0) ++*skipped;
     return true;
 }
@@ -252,7 +253,7 @@ __device__ __forceinline__ bool update_skipped(const int* status, int* skipped, 
 __global__ void adam_kernel(float* __restrict__ w, __nv_bfloat16* __restrict__ wb, const float* __restrict__ g,
                             float* __restrict__ m, float* __restrict__ v, long long n, float lr, float b1, float b2,
                             float eps, float c1, float c2, const int* __restrict__ status, int* __restrict__ skipped) {
-    if (update_skipped(status, skipped, true)) return;
+    if (update_skipped(*status, skipped, true)) return;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         const float gi = g[i];
         const float mi = b1 * m[i] + (1.f - b1) * gi;
@@ -857,14 +858,12 @@ __global__ void mlp_pack_kernel(MlpShape s, const float* __restrict__ w, __nv_bf
 struct AdamArgs {
     float lr, b1, b2, eps, c1, c2;
 };
-__device__ __forceinline__ float adam_step(const AdamArgs& ad, float g, float* w, float* m, float* v) {
+__device__ __forceinline__ void adam_step(const AdamArgs& ad, float g, float* w, float* m, float* v) {
     const float mi = ad.b1 * *m + (1.f - ad.b1) * g;
     const float vi = ad.b2 * *v + (1.f - ad.b2) * g * g;
     *m = mi;
     *v = vi;
-    const float wi = *w - ad.lr * (mi / ad.c1) / (sqrtf(vi / ad.c2) + ad.eps);
-    *w = wi;
-    return wi;
+    *w = *w - ad.lr * (mi / ad.c1) / (sqrtf(vi / ad.c2) + ad.eps);
 }
 __global__ void __launch_bounds__(256) mlp_update_kernel(MlpShape s, const float* __restrict__ dw,
                                                          const float* __restrict__ bgrad,
@@ -873,7 +872,8 @@ __global__ void __launch_bounds__(256) mlp_update_kernel(MlpShape s, const float
                                                          __nv_bfloat16* __restrict__ wp, float* __restrict__ m,
                                                          float* __restrict__ v, float* __restrict__ loss, AdamArgs ad,
                                                          const int* __restrict__ status, int* __restrict__ skipped) {
-    if (update_skipped(status, skipped, ad.lr > 0.f)) return;
+    const int ran_out = *status;
+    const bool training = ad.lr > 0.f;
     const int tiles = s.KT + 2 + s.NT;
     if ((int)blockIdx.x < 8 * tiles) {
         const int tile = blockIdx.x >> 3;
@@ -886,17 +886,31 @@ __global__ void __launch_bounds__(256) mlp_update_kernel(MlpShape s, const float
         float g[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) g[j] = dw[(size_t)tile * kBlk + (c0 + j) * 128 + r];
-        float wi[8];
+        float wi[8], mi[8], vi[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            wi[j] = 0.f;
-            if (k0 + j < in) {
+            wi[j] = mi[j] = vi[j] = 0.f;
+            if (training && k0 + j < in) {
                 const long long i = wo + (long long)(k0 + j) * out + n;
-                grads[i] = g[j];
-                if (ad.lr > 0.f) wi[j] = adam_step(ad, g[j], w + i, m + i, v + i);
+                wi[j] = w[i];
+                mi[j] = m[i];
+                vi[j] = v[i];
             }
         }
-        if (ad.lr > 0.f) {
+        if (update_skipped(ran_out, skipped, training)) return;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            if (k0 + j >= in) continue;
+            const long long i = wo + (long long)(k0 + j) * out + n;
+            grads[i] = g[j];
+            if (training) {
+                adam_step(ad, g[j], wi + j, mi + j, vi + j);
+                w[i] = wi[j];
+                m[i] = mi[j];
+                v[i] = vi[j];
+            }
+        }
+        if (training) {
             __nv_bfloat162 p[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) p[j] = __floats2bfloat162_rn(wi[2 * j], wi[2 * j + 1]);
@@ -908,6 +922,7 @@ __global__ void __launch_bounds__(256) mlp_update_kernel(MlpShape s, const float
         if (threadIdx.x >= 32) return;
         float t = 0.f;
         for (int i = threadIdx.x; i < nloss; i += 32) t += lossp[i];
+        if (ran_out) return;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
         if (threadIdx.x == 0) *loss = t;
@@ -918,8 +933,9 @@ __global__ void __launch_bounds__(256) mlp_update_kernel(MlpShape s, const float
     const int l = min(q >> 7, 3), n = q - l * 128;
     const long long i = (l == 0 ? s.boff[0] : (l == 1 ? s.boff[1] : (l == 2 ? s.boff[2] : s.boff[3]))) + n;
     const float g = bgrad[q];
+    if (ran_out) return;
     grads[i] = g;
-    if (ad.lr > 0.f) adam_step(ad, g, w + i, m + i, v + i);
+    if (training) adam_step(ad, g, w + i, m + i, v + i);
 }
 
 int grid1(long long n) { return (int)std::min<long long>((n + 255) / 256, 148LL * 8); }
@@ -989,7 +1005,8 @@ int mlp_finish(edus_mlp* m, float* loss_host) {
     MCU(m, cudaStreamSynchronize(m->stream));
     if (loss_host) *loss_host = m->report->loss;
     if (m->report->status) {
-        m->step -= m->report->skipped;
+        // every step since the wait ran out was left out, those before a new set of parameters among them
+        m->step = std::max(0, m->step - m->report->skipped);
         MCU(m, cudaMemset(m->status, 0, 2 * sizeof(int)));
         return mfail(m, EDUS_ERR_TIMEOUT,
                      "a bounded wait of a network kernel ran out; training steps left out, weights as before them: " +
@@ -1239,7 +1256,6 @@ int edus_mlp_set_params(edus_mlp* m, const float* host) {
     else to_bf16_kernel<<<grid1(m->nparams), 256, 0, m->stream>>>(m->params, m->wbf, m->nparams);
     MCU(m, cudaMemsetAsync(m->m, 0, m->nparams * sizeof(float), m->stream));
     MCU(m, cudaMemsetAsync(m->v, 0, m->nparams * sizeof(float), m->stream));
-    MCU(m, cudaMemsetAsync(m->skipped, 0, sizeof(int), m->stream));  // steps before the new start
     m->step = 0;
     MCU(m, cudaStreamSynchronize(m->stream));
     return EDUS_OK;

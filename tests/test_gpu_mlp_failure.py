@@ -44,3 +44,34 @@ def test_timed_out_step_changes_nothing_and_is_reported(pkg, hidden, n_out, batc
     net.train_step(x, t, 1e-3)
     ref.train_step(x, t, 1e-3)
     assert np.array_equal(net.params(), ref.params())
+
+
+def test_parameters_set_while_a_timeout_is_pending(pkg):
+    """Steps since a wait ran out are left out until that is reported, also after new parameters; the
+    step count then is that of the new parameters: none."""
+    import torch
+
+    E = pkg.edus
+    rng = np.random.default_rng(8)
+    x = torch.as_tensor(rng.normal(size=(200, 24)).astype(np.float32), device="cuda")
+    t = torch.as_tensor(rng.normal(size=(200, 19)).astype(np.float32), device="cuda")
+    torch.cuda.synchronize()
+    net, ref = (pkg.surrogate.MLP(24, 19, seed=3) for _ in range(2))
+
+    def unread_step(m):
+        assert m._L.edus_mlp_train_step(m._h, 200, ctypes.c_void_p(x.data_ptr()), ctypes.c_void_p(t.data_ptr()),
+                                        ctypes.c_float(1e-3), None) == 0
+
+    start = net.params()
+    net.set_wait_limit(0)
+    for _ in range(3):
+        unread_step(net)
+    net.set_wait_limit(-1)
+    net.set_params(start)
+    unread_step(net)
+    with pytest.raises(E.EdusError):
+        net.params()
+    assert np.array_equal(net.params(), start)
+    for m in (net, ref):
+        m.train_step(x, t, 1e-3)
+    assert np.array_equal(net.params(), ref.params())
